@@ -70,6 +70,8 @@ class MixedPolymul:
             g["engine"] = Engine(kmax, 1, nphi, 256, lr)
             if lc:
                 g["engine"].set_plan(lr, lc)
+                if mode == "graph":
+                    g["engine"].set_tensor(1)
             rids, row = [], 0
             for i in g["inst"]:
                 k = self.specs[i][1]

@@ -104,6 +104,7 @@ int finish_engine(cp_engine** out, cp_engine* h, int log_radix) {
     e.plan_narrow = make_plan(e.logN, 2, e.logN - 2);
     e.narrow_units = 16;
   }
+  e.tensor = log_radix == 0 ? 1 : 0;  // an explicit radix asks for the CUDA-core kernels
   int rc = build_tables_nothrow(e);
   if (rc) {
     delete h;
@@ -215,8 +216,21 @@ int cp_engine_set_plan(cp_engine* h, int log_radix, int log_cta) {
   const int cluster = e.plan.cluster;  // the split-stage form survives a plan change
   e.plan = make_plan(e.logN, log_radix ? log_radix : 3, lc);
   e.plan.cluster = cluster;
+  e.tensor = 0;  // the plan is one of the CUDA-core kernels
   return build_tables_nothrow(e);
 }
+
+int cp_engine_set_tensor(cp_engine* h, int mode) {
+  CP_REQUIRE(h, "cp_engine_set_tensor: NULL engine");
+  CP_REQUIRE(mode >= 0 && mode <= 2, "cp_engine_set_tensor: mode must be 0, 1 or 2");
+  Engine& e = h->e;
+  cudaDeviceSynchronize();
+  e.tensor = mode;
+  free_tables(e);
+  return build_tables_nothrow(e);
+}
+
+int cp_engine_get_tensor(const cp_engine* h) { return h ? (h->e.d_ttab ? 1 : 0) : -1; }
 
 int cp_engine_set_narrow_plan(cp_engine* h, int log_radix, int log_cta, long long max_units) {
   CP_REQUIRE(h, "cp_engine_set_narrow_plan: NULL engine");

@@ -3,6 +3,7 @@
 // 1069-1094).
 #include "dgt_kernels.cuh"
 #include "launch.cuh"
+#include "tdgt.cuh"
 
 namespace cpoly {
 
@@ -202,6 +203,23 @@ namespace {
 // then the split stage.  With the cluster form the split stage runs inside the kernel.
 int run_transform(const Engine& e, ulonglong2* data, const ulonglong2* fsrc, const InvSrc& isrc, int nres,
                   int rid_off, int npolys, long long poly_stride, bool inverse, cudaStream_t st, const int* rid_list) {
+  if (e.d_ttab && !(rid_list && e.tlayout.S > 0) && (long long)npolys * nres > e.tensor_above) {
+    if (inverse && isrc.untwist > 2) {
+      set_error("dgt: unknown untwist table");
+      return 1;
+    }
+    if (e.tlayout.S == 0)
+      return launch_tdgt(e, data, fsrc, isrc, nres, rid_off, npolys, poly_stride, inverse, st, rid_list);
+    if (!inverse) {
+      if (int rc = launch_split(e, e.plan, e.layout, data, fsrc, nres, rid_off, npolys, poly_stride, false, st))
+        return rc;
+      return launch_tdgt(e, data, nullptr, isrc, nres, rid_off, npolys, poly_stride, false, st, nullptr);
+    }
+    DgtTableLayout L = e.layout;
+    if (isrc.untwist > 0) L.off_untwist = L.off_untwist_pre[isrc.untwist - 1];
+    if (int rc = launch_tdgt(e, data, nullptr, isrc, nres, rid_off, npolys, poly_stride, true, st, nullptr)) return rc;
+    return launch_split(e, e.plan, L, data, nullptr, nres, rid_off, npolys, poly_stride, true, st);
+  }
   const PlanSel ps = select_plan(e, (long long)npolys * nres);
   const DgtPlan& P = ps.P;
   DgtTableLayout Lsel = ps.L;

@@ -67,6 +67,16 @@ struct DgtArgs {
   const int* rid_list;     // work list: residue i of the data uses engine prime rid_list[i] (nullptr: base order)
 };
 
+// Tensor-core DGT tables (tdgt.cu): byte offsets inside one residue's block.  The matrices are
+// stored as the tensor core reads them, [K chunk of 16 bytes][column][16 bytes].
+struct TdgtLayout {
+  int logNc = 0;             // element block: 2^logNc elements, logNc in [10, 13]; 0: no such tables
+  int S = 0;                 // split bits left to the split stage (then the tables carry no twist)
+  size_t f_b1 = 0, f_b2 = 0, f_b3 = 0, f_t1 = 0, f_t2 = 0;            // forward
+  size_t i_b1 = 0, i_b2[3] = {0, 0, 0}, i_b3 = 0, i_t1 = 0, i_t2 = 0; // inverse; i_b2: per InvSrc::untwist
+  size_t stride = 0;         // bytes per residue block
+};
+
 // Where the inverse DGT reads its input.
 //  mode 0: p[0] (same layout as the output; p[0] == output for in place);
 //  mode 1: the BFV tensor product of two ciphertexts (a0, a1) x (b0, b1) =
@@ -124,6 +134,11 @@ struct Engine {
   ModConst* d_mc = nullptr;
   ulonglong2* d_tab = nullptr;     // (k + kl) residue blocks
   uint64_t* d_hps = nullptr;       // packed HPS/MRC constants
+  TdgtLayout tlayout;
+  uint8_t* d_ttab = nullptr;       // tensor-core DGT tables, (k + kl) blocks (nullptr: none)
+  int tensor = 1;                  // transforms on the tensor cores: 0 never, 1 in launches of more than
+                                   // tensor_above residue transforms, 2 always (cp_engine_set_tensor)
+  int tensor_above = 0;
   size_t hps_words = 0;
   // word offsets inside d_hps
   struct HpsOffsets {
@@ -185,6 +200,7 @@ const char* last_error();
 
 // table construction (tables.cu)
 int build_tables(Engine& e);
+int build_tensor_tables(Engine& e);  // tdgt_tables.cu; after the plans are placed
 void free_tables(Engine& e);
 
 }  // namespace cpoly

@@ -263,6 +263,24 @@ inline uint64_t h_invmod(uint64_t a, uint64_t p) { return h_powmod(a, p - 2, p);
 inline uint64_t h_shoup(uint64_t w, uint64_t p) {
   return (uint64_t)(((unsigned __int128)w << 64) / p);
 }
+// h_mulmod and h_shoup for the primes p = 2^63 - c of the table (m.pm), by folds in place of
+// 128-bit divisions; other primes take the divisions.
+inline uint64_t h_mul(uint64_t a, uint64_t b, const ModConst& m) {
+  return m.pm ? mul_mod(a, b, m) : h_mulmod(a, b, m.p);
+}
+inline uint64_t h_shoup(uint64_t w, const ModConst& m) {
+  if (!m.pm) return h_shoup(w, m.p);
+  // w 2^64 = 2 w p + 2 w c; floor(2 w c / p) from 2 w c = e 2^63 + r = e p + (e c + r), e < 2^32
+  const uint64_t c = (1ull << 63) - m.p;
+  const unsigned __int128 t = (unsigned __int128)(2 * c) * w;
+  const uint64_t e = (uint64_t)(t >> 63), r = (uint64_t)t & 0x7FFFFFFFFFFFFFFFull;
+  uint64_t x = e * c + r, q = 2 * w + e;
+  while (x >= m.p) {
+    x -= m.p;
+    ++q;
+  }
+  return q;
+}
 inline ModConst h_modconst(uint64_t p) {
   ModConst m;
   m.p = p;

@@ -201,6 +201,36 @@ static int place_plan(const DgtPlan& P, int N, DgtTableLayout& L, int off) {
   return off;
 }
 
+// Per-residue factors of the prescaled untwist tables (off_untwist_pre):
+//   Q residue i: (Q/q_i)^-1 and t (Q/q_i)^-1 mod q_i;  B residue j: t Q^-1 (B/b_j)^-1 mod b_j and 1.
+void prescale_factors(const Engine& e, std::vector<uint64_t>& pre0, std::vector<uint64_t>& pre1) {
+  const int nres = e.k + e.kl;
+  pre0.assign(nres, 1);
+  pre1.assign(nres, 1);
+  for (int r = 0; r < nres; ++r) {
+    const uint64_t p = e.primes[r];
+    const bool in_q = r < e.k;
+    const int lo = in_q ? 0 : e.k, hi = in_q ? e.k : nres;
+    uint64_t hat = 1 % p;  // S / s_r mod s_r, S the product of r's base
+    for (int u = lo; u < hi; ++u)
+      if (u != r) hat = h_mulmod(hat, e.primes[u] % p, p);
+    const uint64_t hinv = h_invmod(hat, p), tp = e.t % p;
+    if (in_q) {
+      pre0[r] = hinv;
+      pre1[r] = h_mulmod(tp, hinv, p);
+    } else {
+      uint64_t qm = 1 % p;
+      for (int u = 0; u < e.k; ++u) qm = h_mulmod(qm, e.primes[u] % p, p);
+      pre0[r] = h_mulmod(h_mulmod(tp, h_invmod(qm, p), p), hinv, p);
+    }
+  }
+}
+
+// f(i, arg) for i in [0, n) on the host's threads (shared with tdgt_tables.cu).
+void parallel_for_host(int n, void (*f)(int, void*), void* arg) {
+  parallel_for(n, [&](int i) { f(i, arg); });
+}
+
 int build_tables(Engine& e) {
   const int nres = e.k + e.kl;
   const int N = e.N;
@@ -226,30 +256,13 @@ int build_tables(Engine& e) {
   L2.off_untwist_pre[1] = L.off_untwist_pre[1];
   L2.stride = L.stride;
 
-  // Per-residue factors of the prescaled untwist tables (off_untwist_pre):
-  //   Q residue i: (Q/q_i)^-1 and t (Q/q_i)^-1 mod q_i;  B residue j: t Q^-1 (B/b_j)^-1 mod b_j and 1.
-  std::vector<uint64_t> pre0(nres, 1), pre1(nres, 1);
-  for (int r = 0; r < nres; ++r) {
-    const uint64_t p = e.primes[r];
-    const bool in_q = r < e.k;
-    const int lo = in_q ? 0 : e.k, hi = in_q ? e.k : nres;
-    uint64_t hat = 1 % p;  // S / s_r mod s_r, S the product of r's base
-    for (int u = lo; u < hi; ++u)
-      if (u != r) hat = h_mulmod(hat, e.primes[u] % p, p);
-    const uint64_t hinv = h_invmod(hat, p), tp = e.t % p;
-    if (in_q) {
-      pre0[r] = hinv;
-      pre1[r] = h_mulmod(tp, hinv, p);
-    } else {
-      uint64_t qm = 1 % p;
-      for (int u = 0; u < e.k; ++u) qm = h_mulmod(qm, e.primes[u] % p, p);
-      pre0[r] = h_mulmod(h_mulmod(tp, h_invmod(qm, p), p), hinv, p);
-    }
-  }
+  std::vector<uint64_t> pre0, pre1;
+  prescale_factors(e, pre0, pre1);
 
   std::vector<ulonglong2> tab((size_t)L.stride * nres);
   parallel_for(nres, [&](int r) {
     const uint64_t p = e.primes[r];
+    const ModConst& mc = e.mconst[r];
     ulonglong2* T = tab.data() + (size_t)r * L.stride;
     const uint64_t gen = e.roots[r];
     const uint64_t wN = omega(p, gen, (uint64_t)N);
@@ -258,10 +271,10 @@ int build_tables(Engine& e) {
     std::vector<uint64_t> pw(N), pwi(N);
     pw[0] = pwi[0] = 1;
     for (int i = 1; i < N; ++i) {
-      pw[i] = h_mulmod(pw[i - 1], wN, p);
-      pwi[i] = h_mulmod(pwi[i - 1], wNi, p);
+      pw[i] = h_mul(pw[i - 1], wN, mc);
+      pwi[i] = h_mul(pwi[i - 1], wNi, mc);
     }
-    auto put = [&](int idx, uint64_t w) { T[idx] = make_ulonglong2(w, h_shoup(w, p)); };
+    auto put = [&](int idx, uint64_t w) { T[idx] = make_ulonglong2(w, h_shoup(w, mc)); };
     auto fill_plan = [&](const DgtPlan& P, const DgtTableLayout& Lp) {
       const int R = 1 << P.logR;
       const int Nc = 1 << P.logNc;
@@ -302,17 +315,22 @@ int build_tables(Engine& e) {
     // products per Gaussian element instead of four.
     auto put_gauss = [&](int idx, G w) {
       put(idx, w.re);
-      put(idx + 1, (w.im + p - w.re) % p);
-      put(idx + 2, (uint64_t)(((unsigned __int128)w.re + w.im) % p));
+      put(idx + 1, sub_mod(w.im, w.re, p));
+      put(idx + 2, add_mod(w.re, w.im, p));
+    };
+    auto mulg = [&](G x, G y) {
+      G z;
+      gi_mul(z.re, z.im, x.re, x.im, y.re, y.im, mc);
+      return z;
     };
     const uint64_t f0 = pre0[r], f1 = pre1[r];
     for (int n = 0; n < N; ++n) {
       put_gauss(L.off_twist + 3 * n, a);
       put_gauss(L.off_untwist + 3 * n, b);
-      put_gauss(L.off_untwist_pre[0] + 3 * n, G{h_mulmod(b.re, f0, p), h_mulmod(b.im, f0, p)});
-      put_gauss(L.off_untwist_pre[1] + 3 * n, G{h_mulmod(b.re, f1, p), h_mulmod(b.im, f1, p)});
-      a = gmul(a, xi, p);
-      b = gmul(b, xii, p);
+      put_gauss(L.off_untwist_pre[0] + 3 * n, G{h_mul(b.re, f0, mc), h_mul(b.im, f0, mc)});
+      put_gauss(L.off_untwist_pre[1] + 3 * n, G{h_mul(b.re, f1, mc), h_mul(b.im, f1, mc)});
+      a = mulg(a, xi);
+      b = mulg(b, xii);
     }
   });
 
@@ -632,6 +650,10 @@ int build_tables(Engine& e) {
     free_tables(e);
     return 2;
   }
+  if (const int rc = build_tensor_tables(e)) {
+    free_tables(e);
+    return rc;
+  }
   return 0;
 }
 
@@ -640,6 +662,8 @@ void free_tables(Engine& e) {
   if (e.d_mc) cudaFree(e.d_mc);
   if (e.d_hps) cudaFree(e.d_hps);
   if (e.d_err) cudaFree(e.d_err);
+  if (e.d_ttab) cudaFree(e.d_ttab);
+  e.d_ttab = nullptr;
   e.d_err = nullptr;
   e.d_tab = nullptr;
   e.d_mc = nullptr;

@@ -101,13 +101,13 @@ class Engine:
         if not torch.cuda.is_available():
             raise RuntimeError("cupoly_b200 needs a CUDA device")
         _lib.lib()
-        log_cta, split_mode, narrow = 0, 0, None
+        log_cta, split_mode, narrow, tuned_radix = 0, 0, None, 0
         if log_radix == 0:  # use the autotuner's plans for this GPU and size when cached
             from .autotune import cached_narrow_plan, cached_plan, cached_split_mode
 
-            log_radix, log_cta = cached_plan(nphi)
+            tuned_radix, log_cta = cached_plan(nphi)
             split_mode = cached_split_mode(nphi)
-            if log_radix:  # a tuned entry replaces the library's default small-launch plan
+            if tuned_radix:  # a tuned entry replaces the library's default small-launch plan
                 narrow = cached_narrow_plan(nphi)
         h = C.c_void_p()
         if ckks_prec:
@@ -116,14 +116,18 @@ class Engine:
         else:
             call("cp_engine_create", C.byref(h), k, kl, nphi, t, log_radix)
         self.ckks_prec = ckks_prec
-        if log_cta:
-            call("cp_engine_set_plan", h, log_radix, log_cta)
+        self._h = h
+        plan, small = self.get_plan(), self.get_narrow_plan()
+        logN = (nphi // 2).bit_length() - 1
+        if tuned_radix and (plan["log_radix"], plan["log_cta"]) != (min(tuned_radix, logN), min(log_cta or 13, logN)):
+            call("cp_engine_set_plan", h, tuned_radix, log_cta)
+            call("cp_engine_set_tensor", h, 1)  # the tuned CUDA-core plan serves what the tensor cores do not
         if split_mode:
             call("cp_engine_set_split_mode", h, split_mode)
-        if narrow is not None:
+        if narrow is not None and narrow != (small["log_radix"], small["log_cta"], small["max_units"]) and \
+                (narrow[2] or small["max_units"]):
             call("cp_engine_set_narrow_plan", h, narrow[0], narrow[1], narrow[2])
-        self.log_radix = log_radix
-        self._h = h
+        self.log_radix = log_radix or tuned_radix
         self.k = k
         self.kl = kl if kl > 0 else k + 1
         self.nphi = nphi
@@ -142,6 +146,14 @@ class Engine:
         """Register radix 2^log_radix and in-CTA size 2^log_cta (0: 2^13); rebuilds the tables."""
         call("cp_engine_set_plan", self._h, log_radix, log_cta)
         self.log_radix = log_radix
+
+    def set_tensor(self, mode: int):
+        """Transforms on the tensor cores in launches large enough to gain (1, the default), in
+        every launch (2) or never (0); same results.  set_plan selects 0; rebuilds the tables."""
+        call("cp_engine_set_tensor", self._h, int(mode))
+
+    def get_tensor(self) -> bool:
+        return _lib.lib().cp_engine_get_tensor(self._h) == 1
 
     def set_split_mode(self, mode: int):
         """0: split stage as its own kernel (HBM pass); 1: inside a thread-block cluster (DSMEM)."""

@@ -92,6 +92,14 @@ int cp_engine_ckks_prec(const cp_engine* e);
  * stage.  Rebuilds the engine's tables (synchronises the device).  The autotuner
  * (cupoly_b200/autotune.py) measures the candidates and caches the fastest. */
 int cp_engine_set_plan(cp_engine* e, int log_radix, int log_cta);
+
+/* Transforms on the tensor cores (BFV engines, nphi 2048 .. 65536; results are identical): 1, the
+ * default of an engine created with log_radix 0: in launches large enough to gain from them;
+ * 2: in every launch; 0: never.  cp_engine_set_plan selects 0.  Rebuilds the engine's tables
+ * (synchronises the device). */
+int cp_engine_set_tensor(cp_engine* e, int mode);
+/* 1: the engine holds tensor-core tables; 0: it does not; -1: NULL engine. */
+int cp_engine_get_tensor(const cp_engine* e);
 int cp_engine_get_plan(const cp_engine* e, int* log_radix, int* log_cta, int* split_bits);
 /* Second DGT plan for small launches (no counterpart in cuPoly): a transform launch of at
  * most max_units residue transforms (polynomials x residues) uses (log_radix, log_cta)
