@@ -652,28 +652,69 @@ int cp_poly_simple_scaling_tdivq(const cp_engine* h, void* out_t, const void* in
   return hps_simple_scaling(e, out_t, ws, st);
 }
 
+// The chain of both multiplication calls over `npairs` pairs of the operands in[0..3] (a0, a1,
+// b0, b1).  X [4][P][k], XB [4][P][kl], CQ [3][P][k] (may be X), CB and U [3][P][kl] are scratch;
+// cq [3][P][k] receives the results over Q in the coefficient domain (may be CQ or X) and is
+// transformed in place, or into outs[0..2] (one polynomial each) when outs is given.
+static int bfv_chain(const Engine& e, const void* const in[4], int npairs, ulonglong2* X, ulonglong2* XB,
+                     ulonglong2* CQ, ulonglong2* CB, ulonglong2* U, ulonglong2* cq, void* const* outs,
+                     cudaStream_t st) {
+  // Every inverse DGT below untwists with a prescaled table (off_untwist_pre), so that it
+  // also applies the first constant product of the conversion that reads its output.
+  // 1. inverse DGT of the four inputs over Q, gathered into X (no copies):
+  //    X = x_i (Q/q_i)^-1 mod q_i
+  InvSrc gather{};
+  for (int v = 0; v < 4; ++v) gather.p[v] = reinterpret_cast<const ulonglong2*>(in[v]);
+  gather.mode = 2;
+  gather.npairs = npairs;
+  gather.untwist = 1;
+  {
+    NvtxRange r("inverse DGT over Q (4P)");
+    CP_TRY(launch_dgt_ex(e, X, nullptr, &gather, CP_QBASE, 4 * npairs, 0, true, st));
+  }
+  // 2. exact Q -> B extension, forward DGT over B
+  {
+    NvtxRange r("Q -> B, forward DGT over B (4P)");
+    CP_TRY(hps_basis_ext_pre(e, XB, X, true, 4 * npairs, st));
+    CP_TRY(launch_dgt(e, XB, CP_BBASE, 4 * npairs, 0, false, st));
+  }
+  // 3. tensor product computed inside the inverse DGTs (Q side from the inputs, B side from
+  //    XB): CQ = t c_i (Q/q_i)^-1 mod q_i, CB = t Q^-1 (B/b_j)^-1 c_j mod b_j
+  InvSrc tq = gather;
+  tq.mode = 1;
+  tq.untwist = 2;
+  NvtxRange r3("tensor products + inverse DGTs (3P over Q and B)");
+  CP_TRY(launch_dgt_ex(e, CQ, nullptr, &tq, CP_QBASE, 3 * npairs, 0, true, st));
+  InvSrc tb{};
+  for (int v = 0; v < 4; ++v) tb.p[v] = XB + (size_t)v * npairs * e.kl * e.N;
+  tb.mode = 1;
+  tb.npairs = npairs;
+  tb.untwist = 1;
+  CP_TRY(launch_dgt_ex(e, CB, nullptr, &tb, CP_BBASE, 3 * npairs, 0, true, st));
+  // 4. round(t X / Q) and B -> Q, then forward DGT of the outputs
+  NvtxRange r4("scale t/Q, B -> Q, forward DGT over Q (3P)");
+  CP_TRY(hps_scale_to_q_pre(e, cq, CQ, CB, U, 3 * npairs, st));
+  if (!outs) return launch_dgt(e, cq, CP_QBASE, 3 * npairs, 0, false, st);
+  return launch_dgt_scatter3(e, outs, cq, CP_QBASE, st);
+}
+
+// One pair: the batched chain's launches on the caller's separate operands and results (12 to 14
+// launches; the composition of the poly_* calls took about 46, which bound the call: 310 us at
+// nphi 8192, k 5).  CQ and the results take the place of X, so the workspace is 4 k + 10 kl.
 int cp_bfv_mul(const cp_engine* h, void* c0, void* c1, void* c2, const void* a0, const void* a1, const void* b0,
                const void* b1, void* ws, void* stream) {
   CP_BFV_ONLY(h, "cp_bfv_mul");
   CP_REQUIRE(h && c0 && c1 && c2 && a0 && a1 && b0 && b1 && ws, "cp_bfv_mul: bad argument");
   NvtxRange range("cp_bfv_mul");
   const Engine& e = h->e;
-  cudaStream_t st = S(stream);
   const size_t qe = (size_t)e.k * e.N, be = (size_t)e.kl * e.N;
-  ulonglong2* w = reinterpret_cast<ulonglong2*>(ws);
-  // layout: xb[4] (B), cb[3] (B), cq[3] (Q), scratch (k + 2 kl)
-  ulonglong2* xb = w;
-  ulonglong2* cb = xb + 4 * be;
-  ulonglong2* cq = cb + 3 * be;
-  ulonglong2* scratch = cq + 3 * qe;
+  ulonglong2* X = reinterpret_cast<ulonglong2*>(ws);
+  ulonglong2* XB = X + 4 * qe;
+  ulonglong2* CB = XB + 4 * be;
+  ulonglong2* U = CB + 3 * be;
   const void* in[4] = {a0, a1, b0, b1};
-  for (int i = 0; i < 4; ++i) CP_TRY(cp_poly_basis_extension_q_to_b(h, xb + i * be, in[i], scratch, stream));
-  CP_TRY(pw_dr2(e, cq, cq + qe, cq + 2 * qe, a0, a1, b0, b1, CP_QBASE, st));
-  CP_TRY(pw_dr2(e, cb, cb + be, cb + 2 * be, xb, xb + be, xb + 2 * be, xb + 3 * be, CP_BBASE, st));
-  void* outs[3] = {c0, c1, c2};
-  for (int i = 0; i < 3; ++i)
-    CP_TRY(cp_poly_complex_scaling_tdivq(h, outs[i], cq + i * qe, cb + i * be, CP_DESTROY_INPUTS, scratch, stream));
-  return CP_OK;
+  void* const outs[3] = {c0, c1, c2};
+  return bfv_chain(e, in, 1, X, XB, X, CB, U, X, outs, S(stream));
 }
 
 size_t cp_bfv_mul_batch_workspace_bytes(const cp_engine* h, int npairs) {
@@ -698,45 +739,8 @@ int cp_bfv_mul_batch(const cp_engine* h, void* c, const void* a0, const void* a1
   ulonglong2* CQ = XB + 4 * P * be;                    // [3][P][k]
   ulonglong2* CB = CQ + 3 * P * qe;                    // [3][P][kl]
   ulonglong2* U = CB + 3 * P * be;                     // [3][P][kl]
-  // Every inverse DGT below untwists with a prescaled table (off_untwist_pre), so that it
-  // also applies the first constant product of the conversion that reads its output.
-  // 1. inverse DGT of the four inputs over Q, gathered into X (no copies):
-  //    X = x_i (Q/q_i)^-1 mod q_i
-  InvSrc gather{};
-  gather.p[0] = reinterpret_cast<const ulonglong2*>(a0);
-  gather.p[1] = reinterpret_cast<const ulonglong2*>(a1);
-  gather.p[2] = reinterpret_cast<const ulonglong2*>(b0);
-  gather.p[3] = reinterpret_cast<const ulonglong2*>(b1);
-  gather.mode = 2;
-  gather.npairs = npairs;
-  gather.untwist = 1;
-  {
-    NvtxRange r("inverse DGT over Q (4P)");
-    CP_TRY(launch_dgt_ex(e, X, nullptr, &gather, CP_QBASE, 4 * npairs, 0, true, st));
-  }
-  // 2. exact Q -> B extension, forward DGT over B
-  {
-    NvtxRange r("Q -> B, forward DGT over B (4P)");
-    CP_TRY(hps_basis_ext_pre(e, XB, X, true, 4 * npairs, st));
-    CP_TRY(launch_dgt(e, XB, CP_BBASE, 4 * npairs, 0, false, st));
-  }
-  // 3. tensor product computed inside the inverse DGTs (Q side from the inputs, B side from
-  //    XB): CQ = t c_i (Q/q_i)^-1 mod q_i, CB = t Q^-1 (B/b_j)^-1 c_j mod b_j
-  InvSrc tq = gather;
-  tq.mode = 1;
-  tq.untwist = 2;
-  NvtxRange r3("tensor products + inverse DGTs (3P over Q and B)");
-  CP_TRY(launch_dgt_ex(e, CQ, nullptr, &tq, CP_QBASE, 3 * npairs, 0, true, st));
-  InvSrc tb{};
-  for (int v = 0; v < 4; ++v) tb.p[v] = XB + v * P * be;
-  tb.mode = 1;
-  tb.npairs = npairs;
-  tb.untwist = 1;
-  CP_TRY(launch_dgt_ex(e, CB, nullptr, &tb, CP_BBASE, 3 * npairs, 0, true, st));
-  // 4. round(t X / Q) and B -> Q, then forward DGT of the outputs
-  NvtxRange r4("scale t/Q, B -> Q, forward DGT over Q (3P)");
-  CP_TRY(hps_scale_to_q_pre(e, c, CQ, CB, U, 3 * npairs, st));
-  return launch_dgt(e, c, CP_QBASE, 3 * npairs, 0, false, st);
+  const void* in[4] = {a0, a1, b0, b1};
+  return bfv_chain(e, in, npairs, X, XB, CQ, CB, U, reinterpret_cast<ulonglong2*>(c), nullptr, st);
 }
 
 int cp_sample(const cp_engine* h, void* out, int base, int kind, uint64_t seed, uint32_t stream_id, int npolys,

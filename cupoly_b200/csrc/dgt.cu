@@ -9,6 +9,13 @@ namespace cpoly {
 
 namespace {
 
+// Input and output of a forward transform: `src` (nullptr: in place), and the places of
+// polynomials 0..2 (scatter[0] nullptr: all at the launch's data).
+struct FwdIO {
+  const ulonglong2* src;
+  ulonglong2* scatter[3];
+};
+
 // Grid of a DGT launch.  When only one CTA fits per SM (N = 8192 in one CTA)
 // the grid is persistent -- one CTA per SM striding over the units, each
 // prefetching its next unit into L2 -- which measured 3-8 % faster on B200;
@@ -30,12 +37,12 @@ unsigned persistent_grid(K kernel, int threads, int smem, std::atomic<int>& resi
 }
 
 template <int LOGNC, int LOGR>
-int run_cta(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglong2* data, const ulonglong2* fsrc,
+int run_cta(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglong2* data, const FwdIO& fio,
             const InvSrc& isrc, int nres, int rid_off, int npolys, long long poly_stride, bool inverse, bool twist,
             cudaStream_t st, const int* rid_list) {
   constexpr int T = (1 << LOGNC) >> LOGR;
   constexpr int smem = dgt_smem_bytes<LOGNC, LOGR>();
-  DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list};
+  DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list, {fio.scatter[0], fio.scatter[1], fio.scatter[2]}};
   const int S = P.S;
   const long long blocks = (long long)npolys * nres << S;
   if (blocks <= 0) return 0;
@@ -48,7 +55,7 @@ int run_cta(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglon
     static std::atomic<int> resident{0};
     if (int rc = ensure_smem(k_dgt_fwd<LOGNC, LOGR>, smem, done)) return rc;
     const unsigned grid = persistent_grid(k_dgt_fwd<LOGNC, LOGR>, T, smem, resident, blocks);
-    k_dgt_fwd<LOGNC, LOGR><<<grid, T, smem, st>>>(data, fsrc, A, nres, rid_off, poly_stride, S, twist ? 1 : 0,
+    k_dgt_fwd<LOGNC, LOGR><<<grid, T, smem, st>>>(data, fio.src, A, nres, rid_off, poly_stride, S, twist ? 1 : 0,
                                                   (unsigned)blocks);
   } else {
     static std::atomic<unsigned long long> done{0};
@@ -61,8 +68,7 @@ int run_cta(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglon
   return check_launch("dgt");
 }
 
-using RunFn = int (*)(const Engine&, const DgtPlan&, const DgtTableLayout&, ulonglong2*, const ulonglong2*,
-                      const InvSrc&, int, int, int, long long, bool, bool, cudaStream_t, const int*);
+using RunFn = int (*)(const Engine&, const DgtPlan&, const DgtTableLayout&, ulonglong2*, const FwdIO&, const InvSrc&, int, int, int, long long, bool, bool, cudaStream_t, const int*);
 
 constexpr int kNoCluster = -1;  // the cluster form cannot be scheduled on this device: use the split kernel
 
@@ -70,12 +76,12 @@ constexpr int kNoCluster = -1;  // the cluster form cannot be scheduled on this 
 // per unit: the cluster's CTAs are the chunks of one residue).  Returns kNoCluster,
 // having launched nothing, when the device cannot co-schedule such a cluster.
 template <int LOGNC, int LOGR, int CL>
-int run_cluster(const Engine& e, const DgtPlan&, const DgtTableLayout& L, ulonglong2* data, const ulonglong2* fsrc,
+int run_cluster(const Engine& e, const DgtPlan&, const DgtTableLayout& L, ulonglong2* data, const FwdIO& fio,
                 const InvSrc& isrc, int nres, int rid_off, int npolys, long long poly_stride, bool inverse, bool,
                 cudaStream_t st, const int* rid_list) {
   constexpr int T = (1 << LOGNC) >> LOGR;
   constexpr int smem = dgt_smem_bytes<LOGNC, LOGR>();
-  DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list};
+  DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list, {fio.scatter[0], fio.scatter[1], fio.scatter[2]}};
   const long long blocks = (long long)npolys * nres << CL;
   if (blocks <= 0) return 0;
   if (blocks > 0x7fffffffLL) {
@@ -111,7 +117,7 @@ int run_cluster(const Engine& e, const DgtPlan&, const DgtTableLayout& L, ulongl
   if (!inverse) {
     if (int rc = ensure_smem(k_dgt_fwd<LOGNC, LOGR, CL>, smem, done_f)) return rc;
     if (!schedulable(k_dgt_fwd<LOGNC, LOGR, CL>, ok_f)) return kNoCluster;
-    err = cudaLaunchKernelEx(&cfg, k_dgt_fwd<LOGNC, LOGR, CL>, data, fsrc, A, nres, rid_off, poly_stride, CL, 1,
+    err = cudaLaunchKernelEx(&cfg, k_dgt_fwd<LOGNC, LOGR, CL>, data, fio.src, A, nres, rid_off, poly_stride, CL, 1,
                              (unsigned)blocks);
   } else {
     if (int rc = ensure_smem(k_dgt_inv<LOGNC, LOGR, CL>, smem, done_i)) return rc;
@@ -134,13 +140,13 @@ RunFn pick_cluster(int logNc, int logR, int S) {
 
 // The plan's split stage inside a cluster, when the plan asks for it and a kernel exists;
 // returns kNoCluster otherwise (nothing launched).
-int try_cluster(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglong2* data, const ulonglong2* fsrc,
+int try_cluster(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglong2* data, const FwdIO& fio,
                 const InvSrc& isrc, int nres, int rid_off, int npolys, long long poly_stride, bool inverse,
                 cudaStream_t st, const int* rid_list) {
   if (!P.cluster || P.S == 0) return kNoCluster;
   RunFn fc = pick_cluster(P.logNc, P.logR, P.S);
   if (!fc) return kNoCluster;
-  return fc(e, P, L, data, fsrc, isrc, nres, rid_off, npolys, poly_stride, inverse, false, st, rid_list);
+  return fc(e, P, L, data, fio, isrc, nres, rid_off, npolys, poly_stride, inverse, false, st, rid_list);
 }
 
 // (logNc, effective logR) -> instantiation.
@@ -157,10 +163,10 @@ RunFn pick(int logNc, int logR) {
   return nullptr;
 }
 
-int launch_split(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglong2* data, const ulonglong2* src,
+int launch_split(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglong2* data, const FwdIO& fio,
                  int nres, int rid_off, int npolys, long long poly_stride, bool inverse, cudaStream_t st,
                  const int* rid_list = nullptr) {
-  DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list};
+  DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list, {fio.scatter[0], fio.scatter[1], fio.scatter[2]}};
   const int Nc = 1 << P.logNc;
   const long long blocks = (long long)npolys * nres * (Nc / 256);
   if (blocks > 0x7fffffffLL) {
@@ -170,9 +176,9 @@ int launch_split(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulo
   const int S = P.S, lc = P.logNc, lr = P.logR;
   if (!inverse) {
     if (S == 1)
-      k_dgt_split<1, false><<<(unsigned)blocks, 256, 0, st>>>(data, src, A, nres, rid_off, poly_stride, lc, lr);
+      k_dgt_split<1, false><<<(unsigned)blocks, 256, 0, st>>>(data, fio.src, A, nres, rid_off, poly_stride, lc, lr);
     else
-      k_dgt_split<2, false><<<(unsigned)blocks, 256, 0, st>>>(data, src, A, nres, rid_off, poly_stride, lc, lr);
+      k_dgt_split<2, false><<<(unsigned)blocks, 256, 0, st>>>(data, fio.src, A, nres, rid_off, poly_stride, lc, lr);
   } else {
     if (S == 1)
       k_dgt_split<1, true><<<(unsigned)blocks, 256, 0, st>>>(data, nullptr, A, nres, rid_off, poly_stride, lc, lr);
@@ -197,28 +203,33 @@ PlanSel select_plan(const Engine& e, long long units) {
 
 namespace {
 
+// Whether a launch of `units` residue transforms runs on the tensor cores.
+bool use_tensor(const Engine& e, long long units, const int* rid_list) {
+  return e.d_ttab && !(rid_list && e.tlayout.S > 0) && units > e.tensor_above;
+}
+
 // One transform of npolys x nres residues with the plan selected for that many units:
 // forward = split stage (when any) then the in-CTA kernel, which also twists when there is
 // no split stage; inverse = the in-CTA kernel (untwisting when there is no split stage)
 // then the split stage.  With the cluster form the split stage runs inside the kernel.
-int run_transform(const Engine& e, ulonglong2* data, const ulonglong2* fsrc, const InvSrc& isrc, int nres,
+int run_transform(const Engine& e, ulonglong2* data, const FwdIO& fio, const InvSrc& isrc, int nres,
                   int rid_off, int npolys, long long poly_stride, bool inverse, cudaStream_t st, const int* rid_list) {
-  if (e.d_ttab && !(rid_list && e.tlayout.S > 0) && (long long)npolys * nres > e.tensor_above) {
+  if (use_tensor(e, (long long)npolys * nres, rid_list)) {
     if (inverse && isrc.untwist > 2) {
       set_error("dgt: unknown untwist table");
       return 1;
     }
     if (e.tlayout.S == 0)
-      return launch_tdgt(e, data, fsrc, isrc, nres, rid_off, npolys, poly_stride, inverse, st, rid_list);
+      return launch_tdgt(e, data, fio.src, isrc, nres, rid_off, npolys, poly_stride, inverse, st, rid_list);
     if (!inverse) {
-      if (int rc = launch_split(e, e.plan, e.layout, data, fsrc, nres, rid_off, npolys, poly_stride, false, st))
+      if (int rc = launch_split(e, e.plan, e.layout, data, fio, nres, rid_off, npolys, poly_stride, false, st))
         return rc;
       return launch_tdgt(e, data, nullptr, isrc, nres, rid_off, npolys, poly_stride, false, st, nullptr);
     }
     DgtTableLayout L = e.layout;
     if (isrc.untwist > 0) L.off_untwist = L.off_untwist_pre[isrc.untwist - 1];
     if (int rc = launch_tdgt(e, data, nullptr, isrc, nres, rid_off, npolys, poly_stride, true, st, nullptr)) return rc;
-    return launch_split(e, e.plan, L, data, nullptr, nres, rid_off, npolys, poly_stride, true, st);
+    return launch_split(e, e.plan, L, data, FwdIO{}, nres, rid_off, npolys, poly_stride, true, st);
   }
   const PlanSel ps = select_plan(e, (long long)npolys * nres);
   const DgtPlan& P = ps.P;
@@ -237,21 +248,22 @@ int run_transform(const Engine& e, ulonglong2* data, const ulonglong2* fsrc, con
     return 3;
   }
   {
-    const int rc = try_cluster(e, P, L, data, fsrc, isrc, nres, rid_off, npolys, poly_stride, inverse, st, rid_list);
+    const int rc = try_cluster(e, P, L, data, fio, isrc, nres, rid_off, npolys, poly_stride, inverse, st, rid_list);
     if (rc != kNoCluster) return rc;
   }
   const int S = P.S;
   if (!inverse) {
     if (S > 0) {
-      int rc = launch_split(e, P, L, data, fsrc, nres, rid_off, npolys, poly_stride, false, st, rid_list);
+      int rc = launch_split(e, P, L, data, fio, nres, rid_off, npolys, poly_stride, false, st, rid_list);
       if (rc) return rc;
-      return fn(e, P, L, data, nullptr, isrc, nres, rid_off, npolys, poly_stride, false, false, st, rid_list);
+      return fn(e, P, L, data, FwdIO{nullptr, {fio.scatter[0], fio.scatter[1], fio.scatter[2]}}, isrc, nres, rid_off,
+                npolys, poly_stride, false, false, st, rid_list);
     }
-    return fn(e, P, L, data, fsrc, isrc, nres, rid_off, npolys, poly_stride, false, true, st, rid_list);
+    return fn(e, P, L, data, fio, isrc, nres, rid_off, npolys, poly_stride, false, true, st, rid_list);
   }
-  int rc = fn(e, P, L, data, nullptr, isrc, nres, rid_off, npolys, poly_stride, true, S == 0, st, rid_list);
+  int rc = fn(e, P, L, data, FwdIO{}, isrc, nres, rid_off, npolys, poly_stride, true, S == 0, st, rid_list);
   if (rc || S == 0) return rc;
-  return launch_split(e, P, L, data, nullptr, nres, rid_off, npolys, poly_stride, true, st, rid_list);
+  return launch_split(e, P, L, data, FwdIO{}, nres, rid_off, npolys, poly_stride, true, st, rid_list);
 }
 
 }  // namespace
@@ -276,7 +288,25 @@ int launch_dgt_ex(const Engine& e, void* dst_v, const void* fsrc_v, const InvSrc
     isrc.mode = 0;
     isrc.npairs = 1;
   }
-  return run_transform(e, data, fsrc, isrc, nres, rid_off, npolys, poly_stride, inverse, st, nullptr);
+  return run_transform(e, data, FwdIO{fsrc, {}}, isrc, nres, rid_off, npolys, poly_stride, inverse, st, nullptr);
+}
+
+int launch_dgt_scatter3(const Engine& e, void* const dst[3], const void* src_v, int base, cudaStream_t st) {
+  const int nres = e.n_residues(base);
+  if (nres < 0 || base == 3) {
+    set_error("dgt: unknown base");
+    return 1;
+  }
+  const ulonglong2* src = reinterpret_cast<const ulonglong2*>(src_v);
+  const long long stride = (long long)nres * e.N;
+  if (use_tensor(e, 3LL * nres, nullptr)) {  // the tensor-core kernel has one output
+    for (int v = 0; v < 3; ++v)
+      if (int rc = launch_dgt_ex(e, dst[v], src + v * stride, nullptr, base, 1, 0, false, st)) return rc;
+    return 0;
+  }
+  FwdIO fio{src, {}};
+  for (int v = 0; v < 3; ++v) fio.scatter[v] = reinterpret_cast<ulonglong2*>(dst[v]);
+  return run_transform(e, fio.scatter[0], fio, InvSrc{}, nres, e.rid_offset(base), 3, stride, false, st, nullptr);
 }
 
 // Residues rid_off .. rid_off + nres - 1 of npolys polynomials (stride poly_stride
@@ -290,7 +320,7 @@ int launch_dgt_part(const Engine& e, void* dst_v, const void* src_v, int rid_off
   isrc.p[0] = src ? src : data;
   isrc.mode = 0;
   isrc.npairs = 1;
-  return run_transform(e, data, src, isrc, nres, rid_off, npolys, poly_stride, inverse, st, nullptr);
+  return run_transform(e, data, FwdIO{src, {}}, isrc, nres, rid_off, npolys, poly_stride, inverse, st, nullptr);
 }
 
 int launch_dgt(const Engine& e, void* data, int base, int npolys, long long poly_stride, bool inverse,
@@ -320,7 +350,7 @@ int launch_dgt_list_ex(const Engine& e, void* data_v, const void* fsrc_v, const 
     isrc.mode = 0;
     isrc.npairs = 1;
   }
-  return run_transform(e, data, fsrc, isrc, 1, 0, nlist, (long long)e.N, inverse, st, rid_list);
+  return run_transform(e, data, FwdIO{fsrc, {}}, isrc, 1, 0, nlist, (long long)e.N, inverse, st, rid_list);
 }
 
 }  // namespace cpoly

@@ -174,6 +174,12 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   }
 }
 
+// Where polynomial `poly` of a forward transform is written (by selects, as inv_src_ptr).
+__device__ __forceinline__ ulonglong2* fwd_dst(const DgtArgs& A, ulonglong2* data, int poly, long long poly_stride) {
+  if (!A.scatter[0]) return data + poly * poly_stride;
+  return poly == 0 ? A.scatter[0] : poly == 1 ? A.scatter[1] : A.scatter[2];
+}
+
 // One middle/late forward pass (I >= 1), full radix 2^LOGR, data in smem.
 template <int LOGNC, int LOGR, int I>
 __device__ __forceinline__ void fwd_passes(ulonglong2* sdat, const ulonglong2* srad, const ulonglong2* stw,
@@ -429,8 +435,9 @@ __global__ void __launch_bounds__((1 << LOGNC) >> LOGR, (dgt_min_blocks<LOGNC, L
   const uint64_t p = A.mc[rid].p;
   const ulonglong2* tab = A.tab + (size_t)rid * A.stride;
   const size_t off = unit_off(ub);
-  ulonglong2* x = data + off;
-  const ulonglong2* xs = in_base + off;
+  const int poly = pr / nres;
+  ulonglong2* x = fwd_dst(A, data, poly, poly_stride) + (off - (size_t)poly * poly_stride);
+  const ulonglong2* xs = src_base ? src_base + off : x;  // in place: the output's own place
   for (int j = tid; j < R; j += T) srad[j] = tab[A.L.off_rad + j];
   stage_twiddles<LOGNC, LOGR>(stw, tab, A.L.off_fwd);
   __syncthreads();
@@ -672,8 +679,8 @@ __global__ void __launch_bounds__(256)
   const int rid = A.rid_list ? A.rid_list[pr] : rid_off + r;
   const uint64_t p = A.mc[rid].p;
   const ulonglong2* tab = A.tab + (size_t)rid * A.stride;
-  ulonglong2* x = data + poly * poly_stride + ((size_t)r << (logNc + S));
-  const ulonglong2* xs = (src_base ? src_base : data) + poly * poly_stride + ((size_t)r << (logNc + S));
+  ulonglong2* x = (INV ? data + poly * poly_stride : fwd_dst(A, data, poly, poly_stride)) + ((size_t)r << (logNc + S));
+  const ulonglong2* xs = src_base ? src_base + poly * poly_stride + ((size_t)r << (logNc + S)) : x;
   constexpr int K = 1 << S;
   uint64_t xr[K], xi[K];
   const int R = 1 << logR;

@@ -65,6 +65,7 @@ struct DgtArgs {
   DgtTableLayout L;
   const ModConst* mc;      // per engine residue
   const int* rid_list;     // work list: residue i of the data uses engine prime rid_list[i] (nullptr: base order)
+  ulonglong2* scatter[3];  // forward output of polynomials 0..2 (scatter[0] nullptr: at `data`)
 };
 
 // Tensor-core DGT tables (tdgt.cu): byte offsets inside one residue's block.  The matrices are
