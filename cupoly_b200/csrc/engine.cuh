@@ -188,11 +188,25 @@ struct Engine {
   } ho{};
   uint64_t t_shoup_one = 0;        // floor(2^64 / t)
   uint64_t h_q_mod_t = 0, h_qinv_t = 0, h_qinv_t_s = 0;  // Q mod t, Q^-1 mod t
+  // byte matrices of the base conversions of prescaled residues (hps.cu): Q -> B, t/Q scaling, B -> Q
+  uint8_t* d_cmat = nullptr;
+  size_t cmat_off[3] = {0, 0, 0};
   int* d_err = nullptr;            // device-side error flag (sampler rejection exhaustion)
   int hps_force_exact = 0;         // 1: every base conversion and scaling takes its exact path (tests)
 
   int n_residues(int base) const;
   int rid_offset(int base) const;
+};
+
+// Byte matrix of a conversion of `ns` residues and one count byte to `ndst` targets: K bytes and
+// columns (8 per target), in groups of an even number of at most 8 targets.
+struct ConvShape {
+  int ns, ndst;
+  __host__ __device__ int kbytes() const { return (8 * ns + 1 + 31) / 32 * 32; }
+  __host__ __device__ int groups() const { return (ndst + 7) / 8; }
+  __host__ __device__ int group() const { return ((ndst + groups() - 1) / groups() + 1) & ~1; }
+  __host__ __device__ int cols() const { return 8 * group() * groups(); }
+  __host__ __device__ int bytes() const { return kbytes() * cols(); }
 };
 
 // thread-local error reporting

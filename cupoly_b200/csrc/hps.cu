@@ -27,8 +27,10 @@
 // the caller applies (1/2 for the centring, 1 - FPERROR for cuPoly's lift; see
 // fast_v).  Otherwise that coefficient takes the exact mixed-radix path, so
 // every result is exact either way.
+#include "byte_sums.cuh"
 #include "launch.cuh"
 #include "pointwise.cuh"
+#include "umma.cuh"
 
 namespace cpoly {
 
@@ -580,6 +582,198 @@ __global__ void __launch_bounds__(128) k_complex_scaling_pre(ulonglong2* __restr
   }
 }
 
+// ---- prescaled conversions on the tensor cores ----
+//
+// The conversions of prescaled inputs are one matrix product: output t = sum_i y_i h_ti - v S.
+// Over bytes (see tdgt.cu) it is an 8-bit matrix product: a coefficient's row holds the 8 bytes
+// of each y_i and the FP64 overflow count v as one more byte, and target t has 8 columns.  What
+// is left per output is the sum of its 8 columns and one fold, in place of a 192-bit dot product
+// and its reduction (for 5 residues about 120 cycles of the integer multiply pipe a warp, now
+// 20).  Bound by HBM and the latency of a tile's steps: at nphi 8192, 128 pairs, Q -> B of 512
+// polynomials 183 -> 99 us, scaling of 384 150 -> 121 us, B -> Q 131 -> 73 us (0.58, 0.55, 0.59 of
+// the measured HBM rate).  A CTA of 128 threads takes 128 elements at a time:
+// thread j loads element j's residues, writes the bytes of its real and imaginary coefficient
+// to row j of two operand tiles, and reads back row j of the two products, `group` targets at a
+// time (128 columns of tensor memory, four CTAs a SM).  A coefficient that the FP64 count cannot
+// decide is computed again on its exact path.
+struct TensorConv {
+  const uint8_t* mat;
+  int tiles_per_poly, ntiles;
+  int* err;
+};
+
+template <int NS>
+constexpr int conv_kbytes() {
+  return (8 * NS + 1 + 31) / 32 * 32;
+}
+
+template <int NS, bool SCALE, class Args>
+__global__ void __launch_bounds__(128, 4)
+    k_conv_tensor(ulonglong2* __restrict__ out, const ulonglong2* __restrict__ in, const ulonglong2* __restrict__ in_b,
+                  const __grid_constant__ Args a, const __grid_constant__ TensorConv tc) {
+  using namespace umma;
+  constexpr int KB = conv_kbytes<NS>(), CH = KB / 16;
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  __shared__ uint64_t s_bar[2];
+  __shared__ uint32_t s_slot;
+  __shared__ int s_fail;
+  const int tid = threadIdx.x;
+  const int ndst = SCALE ? reinterpret_cast<const ScaleArgs&>(a).kl : reinterpret_cast<const ConvArgs&>(a).ndst;
+  const ConvShape sh{NS, ndst};
+  const int grp = sh.group(), ngrp = sh.groups(), cols = sh.cols();
+  const uint32_t sA = smem_u32(smem_raw), sB = sA + 2 * 128 * KB;
+  const uint32_t bD = smem_u32(s_bar), bB = bD + 8;
+  if (tid == 0) {
+    mbar_init(bD, 1);
+    mbar_init(bB, 1);
+    mbar_init_fence();
+    s_fail = 0;
+    mbar_expect_tx(bB, sh.bytes());
+    bulk_load(sB, tc.mat, sh.bytes(), bB);
+  }
+  if (tid < 32) tmem_alloc(smem_u32(&s_slot), 128);
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = s_slot, tl = tmem + ((uint32_t)(tid & 96) << 16);
+  const uint32_t idesc = idesc_u8(128, 8 * grp);
+  const uint64_t dA = smem_desc(sA, 2048, 128, kSwzNone), dB = smem_desc(sB, cols * 16, 128, kSwzNone);
+  uint32_t k8 = 256;
+  asm volatile("" : "+r"(k8));
+  uint32_t pd = 0;
+  int src_off = 0, dst_off = 0, N = 0;
+  long long in_stride = 0, out_stride = 0, b_stride = 0;
+  const ModConst* mc;
+  const uint64_t* invd;
+  int force_exact;
+  if constexpr (SCALE) {
+    dst_off = a.k;
+    N = a.N;
+    in_stride = a.q_stride;
+    b_stride = a.b_stride;
+    out_stride = a.out_stride;
+    mc = a.mc;
+    invd = a.fq.invd;
+    force_exact = a.force_exact;
+  } else {
+    src_off = a.src_off;
+    dst_off = a.dst_off;
+    N = a.N;
+    in_stride = a.in_stride;
+    out_stride = a.out_stride;
+    mc = a.mc;
+    invd = a.f.invd;
+    force_exact = a.force_exact;
+  }
+  (void)src_off;
+  ulonglong2 x[NS];
+  auto load = [&](int tile) {
+    const ulonglong2* p = in + (tile / tc.tiles_per_poly) * in_stride + (tile % tc.tiles_per_poly) * 128 + tid;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) x[i] = p[(size_t)i * N];
+  };
+  constexpr bool kEarly = NS <= 11;  // the next tile's residues in registers during the products
+  if (kEarly && (int)blockIdx.x < tc.ntiles) load(blockIdx.x);
+  bool first = true;
+  for (int tile = blockIdx.x; tile < tc.ntiles; tile += gridDim.x) {
+    if (!kEarly) load(tile);
+    // the overflow counts (fast_v), then both rows
+    uint64_t y[NS];
+    bool ok = !force_exact;
+#pragma unroll
+    for (int comp = 0; comp < 2; ++comp) {
+#pragma unroll
+      for (int i = 0; i < NS; ++i) y[i] = comp ? x[i].y : x[i].x;
+      int v;
+      bool above, neg = false;
+      ok &= SCALE ? fast_v<NS>(y, invd, true, v, above) : fast_v<NS>(y, invd, false, v, above, true, &neg);
+      v += SCALE ? (above ? 1 : 0) : (neg ? 1 : 0);
+      const uint32_t row = sA + comp * 128 * KB + tid * 16;
+#pragma unroll
+      for (int ch = 0; ch < CH; ++ch) {
+        const uint64_t lo = 2 * ch < NS ? y[2 * ch < NS ? 2 * ch : 0] : (2 * ch == NS ? (uint64_t)v : 0);
+        const uint64_t hi = 2 * ch + 1 < NS ? y[2 * ch + 1 < NS ? 2 * ch + 1 : 0] : (2 * ch + 1 == NS ? (uint64_t)v : 0);
+        asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(row + ch * 2048), "l"(lo), "l"(hi) : "memory");
+      }
+    }
+    fence_async_smem();
+    fence_before_sync();
+    __syncthreads();  // every row is written, and the last tile's products are read
+    auto issue = [&](int g) {
+      if (tid == 0) {
+        fence_after_sync();
+#pragma unroll
+        for (int comp = 0; comp < 2; ++comp)
+#pragma unroll
+          for (int ks = 0; ks < KB / 32; ++ks)
+            mma_u8(tmem + 64 * comp, dA + (comp * 128 * KB + ks * 4096) / 16, dB + (ks * 2 * cols + g * grp * 8), idesc,
+                   ks > 0);
+        mma_commit(bD);
+      }
+    };
+    if (first) mbar_wait(bB, 0, &s_fail);
+    first = false;
+    issue(0);
+    const int poly = tile / tc.tiles_per_poly, j = (tile % tc.tiles_per_poly) * 128 + tid;
+    if (kEarly && tile + (int)gridDim.x < tc.ntiles) load(tile + gridDim.x);  // on their way during the products
+    ulonglong2* o = out + poly * out_stride + j;
+    const ulonglong2* ib = SCALE ? in_b + poly * b_stride + j : nullptr;
+    for (int g = 0; g < ngrp; ++g) {
+      const int t0 = g * grp, t1 = t0 + grp < ndst ? t0 + grp : ndst;
+      ulonglong2 bn = make_ulonglong2(0, 0);
+      if (SCALE) bn = ib[(size_t)t0 * N];
+      mbar_wait(bD, pd & 1, &s_fail);
+      ++pd;
+      fence_after_sync();
+      uint32_t c0[16], c1[16];
+      auto ld = [&](int t, uint32_t(&c)[16]) { tmem_ld8x2(c, tl + 8 * (t - t0), tl + 64 + 8 * (t - t0)); };
+      auto one = [&](int t, const uint32_t(&c)[16]) {
+        const ulonglong2 b = bn;
+        if (SCALE && t + 1 < t1) bn = ib[(size_t)(t + 1) * N];
+        const uint64_t p = mc[dst_off + t].p;
+        const Red R{p, (uint32_t)((1ull << 63) - p), k8, k8 << 8};
+        uint64_t re = red2p(col_sum(c, R), p), im = red2p(col_sum(c + 8, R), p);
+        if (SCALE) {
+          re = sub_mod(b.x, re, p);
+          im = sub_mod(b.y, im, p);
+        }
+        o[(size_t)t * N] = make_ulonglong2(re, im);
+      };
+      ld(t0, c0);
+#pragma unroll 1
+      for (int t = t0; t < t1; t += 2) {  // the next target's columns are on their way while one is summed
+        tmem_ld_wait(c0);
+        if (t + 1 < t1) ld(t + 1, c1);
+        one(t, c0);
+        if (t + 1 < t1) {
+          tmem_ld_wait(c1);
+          if (t + 2 < t1) ld(t + 2, c0);
+          one(t + 1, c1);
+        }
+      }
+      if (g + 1 < ngrp) {
+        fence_before_sync();
+        __syncthreads();  // the group's products are read
+        issue(g + 1);
+      }
+    }
+    if (!ok) {
+      uint64_t* ow = reinterpret_cast<uint64_t*>(out + poly * out_stride);
+      const uint64_t* iw = reinterpret_cast<const uint64_t*>(in + poly * in_stride);
+      for (int comp = 0; comp < 2; ++comp) {
+        if constexpr (SCALE)
+          scale_exact_pre_write<NS>(ow, iw, reinterpret_cast<const uint64_t*>(in_b + poly * b_stride), j, comp, a);
+        else
+          ext_exact<NS>(ow, iw, j, comp, a, true);
+      }
+    }
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (tid < 32) tmem_dealloc(tmem, 128);
+  if (tid == 0 && s_fail) atomicExch(tc.err, 2);
+}
+
 struct SimpleArgs {
   const ModConst* mc;
   const uint64_t *inv, *inv_s, *hor, *hor_s, *half, *t_q, *t_q_s;
@@ -665,6 +859,39 @@ int launch_ss_n(ulonglong2* out, const ulonglong2* q, const SimpleArgs& a, cudaS
   return check_launch("simple_scaling");
 }
 
+// Whether `npolys` conversions from `ns` residues run on the tensor cores.  From 4 residues on
+// they are faster at every batch size (whole chain, nphi 8192, us: k 4, 2 pairs 74 -> 71, 256 pairs
+// 2097 -> 1921); with 1 or 2 the dot products are too short to be worth the operand's way through
+// shared memory (k 1, 256 pairs 703 against 766); with 3 they gain in large batches (8 pairs
+// 96.3 against 97.3, 64 pairs 466 -> 447).
+bool conv_on_tensor(const Engine& e, int ns, int npolys) {
+  if (!e.d_cmat || e.N < 128) return false;
+  return ns >= 4 || (ns == 3 && (long long)npolys * e.N >= 1 << 18);
+}
+
+template <int NS, bool SCALE, class Args>
+int launch_conv_tensor(const Engine& e, int which, ulonglong2* out, const ulonglong2* in, const ulonglong2* in_b,
+                       const Args& a, int ndst, int npolys, cudaStream_t st) {
+  static std::atomic<unsigned long long> done{0};
+  const ConvShape sh{NS, ndst};
+  int smem = 2 * 128 * sh.kbytes() + sh.bytes();
+  if (smem < 46 * 1024) smem = 46 * 1024;  // at most four CTAs a SM: each holds 128 columns of tensor memory
+  if (int rc = ensure_smem(k_conv_tensor<NS, SCALE, Args>, 2 * 128 * 224 + 224 * 192, done)) return rc;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long tiles = (long long)npolys * (e.N / 128);
+  if (tiles > 0x3fffffffLL) {
+    set_error("base conversion: batch too large");
+    return CP_ERR_INVALID_;
+  }
+  const int per = smem <= 56 * 1024 ? 4 : (smem <= 75 * 1024 ? 3 : 2);
+  const long long most = (long long)(sms > 0 ? sms : 1) * per;
+  const TensorConv tc{e.d_cmat + e.cmat_off[which], e.N / 128, (int)tiles, e.d_err};
+  k_conv_tensor<NS, SCALE, Args><<<(unsigned)(tiles < most ? tiles : most), 128, smem, st>>>(out, in, in_b, a, tc);
+  return check_launch("base conversion (tensor cores)");
+}
+
 #define CP_SWITCH_NS(n, CALL)                                                                             \
   switch (n) {                                                                                            \
     case 1: return CALL(1); case 2: return CALL(2); case 3: return CALL(3); case 4: return CALL(4);       \
@@ -740,6 +967,11 @@ int hps_basis_ext_pre(const Engine& e, void* out, const void* in, bool q_to_b, i
   const int ns = q_to_b ? e.k : e.kl;
   auto* o = reinterpret_cast<ulonglong2*>(out);
   auto* i = reinterpret_cast<const ulonglong2*>(in);
+  if (conv_on_tensor(e, ns, npolys)) {
+#define CALL(n) (launch_conv_tensor<n, false, ConvArgs>(e, q_to_b ? 0 : 2, o, i, nullptr, a, a.ndst, npolys, st))
+    CP_SWITCH_NS(ns, CALL)
+#undef CALL
+  }
 #define CALL(n) launch_basis_ext_pre_n<n>(o, i, a, npolys, st)
   CP_SWITCH_NS(ns, CALL)
 #undef CALL
@@ -818,9 +1050,15 @@ int hps_scale_to_q_pre(const Engine& e, void* out_q, const void* in_q, const voi
   auto* q = reinterpret_cast<const ulonglong2*>(in_q);
   auto* b = reinterpret_cast<const ulonglong2*>(in_b);
   int rc;
-#define CALL(n) launch_cs_pre_n<n>(o, q, b, a, npolys, st)
-  rc = [&]() -> int { CP_SWITCH_NS(e.k, CALL) }();
+  if (conv_on_tensor(e, e.k, npolys)) {
+#define CALL(n) (launch_conv_tensor<n, true, ScaleArgs>(e, 1, o, q, b, a, e.kl, npolys, st))
+    rc = [&]() -> int { CP_SWITCH_NS(e.k, CALL) }();
 #undef CALL
+  } else {
+#define CALL(n) launch_cs_pre_n<n>(o, q, b, a, npolys, st)
+    rc = [&]() -> int { CP_SWITCH_NS(e.k, CALL) }();
+#undef CALL
+  }
   if (rc) return rc;
   return hps_basis_ext_pre(e, out_q, scratch_b, false, npolys, st);
 }

@@ -650,6 +650,42 @@ int build_tables(Engine& e) {
     free_tables(e);
     return 2;
   }
+  if (!e.ckks_prec) {
+    // conv[target][source] as bytes, and the count's coefficient as source ns: column 8 t + j,
+    // K byte 8 i + b holds byte j of f 2^(8 b) mod m_t (the count has one byte)
+    const ConvShape sh[3] = {{e.k, e.kl}, {e.k, e.kl}, {e.kl, e.k}};
+    const int src[3] = {e.ho.fq_hmod, e.ho.cs_hm2, e.ho.fb_hmod};
+    const int neg[3] = {e.ho.fq_negv, e.ho.cs_negw2, e.ho.fb_negv};
+    size_t total = 0;
+    for (int v = 0; v < 3; ++v) {
+      e.cmat_off[v] = total;
+      total += (sh[v].bytes() + 127) & ~127;
+    }
+    std::vector<uint8_t> cm(total, 0);
+    for (int v = 0; v < 3; ++v)
+      for (int t = 0; t < sh[v].ndst; ++t) {
+        const ModConst& m = e.mconst[v == 2 ? t : e.k + t];
+        for (int i = 0; i <= sh[v].ns; ++i) {
+          uint64_t f = i < sh[v].ns ? H[src[v] + t * sh[v].ns + i] : H[neg[v] + t * (sh[v].ns + 1) + 1];
+          for (int b = 0; b < (i < sh[v].ns ? 8 : 1); ++b) {
+            const int kb = 8 * i + b;
+            uint8_t* at = cm.data() + e.cmat_off[v] + (size_t)(kb >> 4) * sh[v].cols() * 16 + (kb & 15);
+            for (int j = 0; j < 8; ++j) at[(size_t)(8 * t + j) * 16] = (uint8_t)(f >> (8 * j));
+            f = h_mul(f, 256, m);
+          }
+        }
+      }
+    if ((err = cudaMalloc(&e.d_cmat, cm.size())) != cudaSuccess) {
+      set_error(std::string("cudaMalloc failed for engine tables: ") + cudaGetErrorString(err));
+      free_tables(e);
+      return 4;
+    }
+    if ((err = cudaMemcpy(e.d_cmat, cm.data(), cm.size(), cudaMemcpyHostToDevice)) != cudaSuccess) {
+      set_error(std::string("table upload failed: ") + cudaGetErrorString(err));
+      free_tables(e);
+      return 2;
+    }
+  }
   if (const int rc = build_tensor_tables(e)) {
     free_tables(e);
     return rc;
@@ -664,6 +700,8 @@ void free_tables(Engine& e) {
   if (e.d_err) cudaFree(e.d_err);
   if (e.d_ttab) cudaFree(e.d_ttab);
   e.d_ttab = nullptr;
+  if (e.d_cmat) cudaFree(e.d_cmat);
+  e.d_cmat = nullptr;
   e.d_err = nullptr;
   e.d_tab = nullptr;
   e.d_mc = nullptr;
