@@ -422,9 +422,13 @@ int cp_polymul(const cp_engine* h, void* c, const void* a, const void* b, int ba
   if (int rc = launch_dgt_ex(e, wb, b, nullptr, base, npolys, 0, false, st)) return rc;
   InvSrc is{};
   is.p[0] = wa;
-  is.p[1] = wb;
-  is.mode = 3;
   is.npairs = 1;
+  if (dgt_on_tensor(e, (long long)npolys * e.n_residues(base))) {  // see tensor_inverse
+    if (int rc = pw_mul(e, wa, wa, wb, base, st, npolys, true)) return rc;
+  } else {
+    is.p[1] = wb;
+    is.mode = 3;
+  }
   return launch_dgt_ex(e, c, nullptr, &is, base, npolys, 0, true, st);
 }
 
@@ -438,9 +442,13 @@ int cp_polymul_list(const cp_engine* h, void* c, const void* a, const void* b, v
   if (int rc = launch_dgt_list_ex(e, wb, b, nullptr, rid_list, nlist, false, st)) return rc;
   InvSrc is{};
   is.p[0] = reinterpret_cast<const ulonglong2*>(wa);
-  is.p[1] = reinterpret_cast<const ulonglong2*>(wb);
-  is.mode = 3;
   is.npairs = 1;
+  if (dgt_on_tensor(e, nlist, true)) {  // see tensor_inverse
+    if (int rc = pw_mul_list(e, wa, wa, wb, rid_list, nlist, st, true)) return rc;
+  } else {
+    is.p[1] = reinterpret_cast<const ulonglong2*>(wb);
+    is.mode = 3;
+  }
   return launch_dgt_list_ex(e, c, nullptr, &is, rid_list, nlist, true, st);
 }
 
@@ -652,6 +660,29 @@ int cp_poly_simple_scaling_tdivq(const cp_engine* h, void* out_t, const void* in
   return hps_simple_scaling(e, out_t, ws, st);
 }
 
+// out [3][npairs] = the inverse DGTs of c0, c1, c2 of npairs pairs of p = {a0, a1, b0, b1} over
+// `base`, with untwist table `untwist`.  On the CUDA cores the products are formed while the
+// transform loads; a tensor-core unit would wait for them (its loads are on its critical path), so
+// there a streaming kernel forms them first (nphi 8192, k 5, 128 pairs over Q and B: 486 us fused,
+// 420 us so).
+static int tensor_inverse(const Engine& e, ulonglong2* out, const ulonglong2* const p[4], int base, int npairs,
+                          int untwist, cudaStream_t st) {
+  const int nres = e.n_residues(base);
+  InvSrc is{};
+  is.untwist = untwist;
+  if (dgt_on_tensor(e, 3LL * npairs * nres)) {
+    const size_t one = (size_t)npairs * nres * e.N;
+    CP_TRY(pw_dr2(e, out, out + one, out + 2 * one, p[0], p[1], p[2], p[3], base, st, npairs, true));
+    is.p[0] = out;
+    is.npairs = 1;
+  } else {
+    for (int v = 0; v < 4; ++v) is.p[v] = p[v];
+    is.mode = 1;
+    is.npairs = npairs;
+  }
+  return launch_dgt_ex(e, out, nullptr, &is, base, 3 * npairs, 0, true, st);
+}
+
 // The chain of both multiplication calls over `npairs` pairs of the operands in[0..3] (a0, a1,
 // b0, b1).  X [4][P][k], XB [4][P][kl], CQ [3][P][k] (may be X), CB and U [3][P][kl] are scratch;
 // cq [3][P][k] receives the results over Q in the coefficient domain (may be CQ or X) and is
@@ -678,19 +709,12 @@ static int bfv_chain(const Engine& e, const void* const in[4], int npairs, ulong
     CP_TRY(hps_basis_ext_pre(e, XB, X, true, 4 * npairs, st));
     CP_TRY(launch_dgt(e, XB, CP_BBASE, 4 * npairs, 0, false, st));
   }
-  // 3. tensor product computed inside the inverse DGTs (Q side from the inputs, B side from
-  //    XB): CQ = t c_i (Q/q_i)^-1 mod q_i, CB = t Q^-1 (B/b_j)^-1 c_j mod b_j
-  InvSrc tq = gather;
-  tq.mode = 1;
-  tq.untwist = 2;
+  // 3. tensor products and their inverse DGTs (Q side from the inputs, B side from XB): CQ = t c_i (Q/q_i)^-1 mod q_i, CB = t Q^-1 (B/b_j)^-1 c_j mod b_j
   NvtxRange r3("tensor products + inverse DGTs (3P over Q and B)");
-  CP_TRY(launch_dgt_ex(e, CQ, nullptr, &tq, CP_QBASE, 3 * npairs, 0, true, st));
-  InvSrc tb{};
-  for (int v = 0; v < 4; ++v) tb.p[v] = XB + (size_t)v * npairs * e.kl * e.N;
-  tb.mode = 1;
-  tb.npairs = npairs;
-  tb.untwist = 1;
-  CP_TRY(launch_dgt_ex(e, CB, nullptr, &tb, CP_BBASE, 3 * npairs, 0, true, st));
+  const ulonglong2* ext[4];
+  for (int v = 0; v < 4; ++v) ext[v] = XB + (size_t)v * npairs * e.kl * e.N;
+  CP_TRY(tensor_inverse(e, CQ, gather.p, CP_QBASE, npairs, 2, st));
+  CP_TRY(tensor_inverse(e, CB, ext, CP_BBASE, npairs, 1, st));
   // 4. round(t X / Q) and B -> Q, then forward DGT of the outputs
   NvtxRange r4("scale t/Q, B -> Q, forward DGT over Q (3P)");
   CP_TRY(hps_scale_to_q_pre(e, cq, CQ, CB, U, 3 * npairs, st));

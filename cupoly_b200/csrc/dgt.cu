@@ -203,18 +203,13 @@ PlanSel select_plan(const Engine& e, long long units) {
 
 namespace {
 
-// Whether a launch of `units` residue transforms runs on the tensor cores.
-bool use_tensor(const Engine& e, long long units, const int* rid_list) {
-  return e.d_ttab && !(rid_list && e.tlayout.S > 0) && units > e.tensor_above;
-}
-
 // One transform of npolys x nres residues with the plan selected for that many units:
 // forward = split stage (when any) then the in-CTA kernel, which also twists when there is
 // no split stage; inverse = the in-CTA kernel (untwisting when there is no split stage)
 // then the split stage.  With the cluster form the split stage runs inside the kernel.
 int run_transform(const Engine& e, ulonglong2* data, const FwdIO& fio, const InvSrc& isrc, int nres,
                   int rid_off, int npolys, long long poly_stride, bool inverse, cudaStream_t st, const int* rid_list) {
-  if (use_tensor(e, (long long)npolys * nres, rid_list)) {
+  if (dgt_on_tensor(e, (long long)npolys * nres, rid_list != nullptr)) {
     if (inverse && isrc.untwist > 2) {
       set_error("dgt: unknown untwist table");
       return 1;
@@ -268,6 +263,10 @@ int run_transform(const Engine& e, ulonglong2* data, const FwdIO& fio, const Inv
 
 }  // namespace
 
+bool dgt_on_tensor(const Engine& e, long long units, bool list) {
+  return e.d_ttab && !(list && e.tlayout.S > 0) && units > e.tensor_above;
+}
+
 int launch_dgt_ex(const Engine& e, void* dst_v, const void* fsrc_v, const InvSrc* isrc_p, int base, int npolys,
                   long long poly_stride, bool inverse, cudaStream_t st) {
   if (base == 3) return 0;  // TBase: no transform (cuPoly dgt.cu:1087-1088)
@@ -299,7 +298,7 @@ int launch_dgt_scatter3(const Engine& e, void* const dst[3], const void* src_v, 
   }
   const ulonglong2* src = reinterpret_cast<const ulonglong2*>(src_v);
   const long long stride = (long long)nres * e.N;
-  if (use_tensor(e, 3LL * nres, nullptr)) {  // the tensor-core kernel has one output
+  if (dgt_on_tensor(e, 3LL * nres)) {  // the tensor-core kernel has one output
     for (int v = 0; v < 3; ++v)
       if (int rc = launch_dgt_ex(e, dst[v], src + v * stride, nullptr, base, 1, 0, false, st)) return rc;
     return 0;

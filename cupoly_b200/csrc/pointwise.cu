@@ -8,6 +8,7 @@
 // residue's constants once.
 #include "launch.cuh"
 #include "pointwise.cuh"
+#include "product_sums.cuh"
 
 namespace cpoly {
 
@@ -18,15 +19,18 @@ using u2 = ulonglong2;
 // blockIdx.y enumerates (polynomial, residue) pairs of a densely packed batch.
 template <class F>
 __global__ void __launch_bounds__(256)
-    k_elementwise(F f, int N, int nres, int rid_off, const ModConst* __restrict__ mc, const int* __restrict__ rid_list) {
+    k_elementwise(F f, int N, int rows, int nres, int rid_off, const ModConst* __restrict__ mc,
+                  const int* __restrict__ rid_list) {
   const int y = blockIdx.y + blockIdx.z * gridDim.y;
+  if (y >= rows) return;
   const ModConst m = mc[rid_list ? rid_list[y] : rid_off + y % nres];
   const size_t base = (size_t)y * N;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < N; j += gridDim.x * blockDim.x) f(base + j, m);
 }
 
 template <class F>
-int launch_ew(const Engine& e, F f, int base, cudaStream_t st, int npolys = 1, const int* rid_list = nullptr) {
+int launch_ew(const Engine& e, F f, int base, cudaStream_t st, int npolys = 1, const int* rid_list = nullptr,
+              bool any_rows = false) {
   const int nres = rid_list ? 1 : e.n_residues(base);
   if (nres <= 0) {
     set_error("pointwise: unknown base");
@@ -38,6 +42,14 @@ int launch_ew(const Engine& e, F f, int base, cudaStream_t st, int npolys = 1, c
   if (bx > 4096) bx = 4096;
   const long long rows = (long long)nres * npolys;
   int gy = (int)rows, gz = 1;
+  if (rows > 0x3fffffffLL) {
+    set_error("pointwise: batch too large");
+    return CP_ERR_INVALID_;
+  }
+  if (any_rows && rows > 65535) {  // inside composite calls: the last block row may reach past the end
+    gy = 65535;
+    gz = (int)((rows + gy - 1) / gy);
+  }
   while (gy > 65535) {  // split rows over z when needed (rows is a multiple of gz)
     gz *= 2;
     if (rows % gz) {
@@ -47,7 +59,7 @@ int launch_ew(const Engine& e, F f, int base, cudaStream_t st, int npolys = 1, c
     gy = (int)(rows / gz);
   }
   dim3 grid(bx, gy, gz);
-  k_elementwise<<<grid, threads, 0, st>>>(f, e.N, nres, rid_list ? 0 : e.rid_offset(base), e.d_mc, rid_list);
+  k_elementwise<<<grid, threads, 0, st>>>(f, e.N, (int)rows, nres, rid_list ? 0 : e.rid_offset(base), e.d_mc, rid_list);
   return check_launch("pointwise");
 }
 
@@ -76,15 +88,19 @@ struct DoubleAddF {
     c2[i] = make_ulonglong2(add_mod(z.x, w.x, m.p), add_mod(z.y, w.y, m.p));
   }
 };
+// The Gaussian product by the prime's form (uniform within a block).
+__device__ __forceinline__ u2 mul_gi(u2 x, u2 y, const ModConst& m) {
+  uint64_t r, im;
+  if (m.pm)
+    gi_mul_pm(r, im, x, y, m.p, (uint32_t)((1ull << 63) - m.p));
+  else
+    gi_mul(r, im, x.x, x.y, y.x, y.y, m);
+  return make_ulonglong2(r, im);
+}
 struct MulF {
   u2* c;
   const u2 *a, *b;
-  __device__ void operator()(size_t i, const ModConst& m) const {
-    const u2 x = a[i], y = b[i];
-    uint64_t r, im;
-    gi_mul(r, im, x.x, x.y, y.x, y.y, m);
-    c[i] = make_ulonglong2(r, im);
-  }
+  __device__ void operator()(size_t i, const ModConst& m) const { c[i] = mul_gi(a[i], b[i], m); }
 };
 struct MulU64F {
   u2* c;
@@ -100,10 +116,8 @@ struct MulAddF {
   u2* d;
   const u2 *a, *b, *c;
   __device__ void operator()(size_t i, const ModConst& m) const {
-    const u2 x = a[i], y = b[i], z = c[i];
-    uint64_t r, im;
-    gi_mul(r, im, x.x, x.y, y.x, y.y, m);
-    d[i] = make_ulonglong2(add_mod(r, z.x, m.p), add_mod(im, z.y, m.p));
+    const u2 z = c[i], r = mul_gi(a[i], b[i], m);
+    d[i] = make_ulonglong2(add_mod(r.x, z.x, m.p), add_mod(r.y, z.y, m.p));
   }
 };
 struct Dr2F {
@@ -111,6 +125,26 @@ struct Dr2F {
   const u2 *c01, *c02, *c11, *c12;
   __device__ void operator()(size_t i, const ModConst& m) const {
     const u2 a0 = c01[i], a1 = c02[i], b0 = c11[i], b1 = c12[i];
+    if (m.pm) {  // c1's two products in one sum each: below 4 p^2 < 2^128
+      const uint64_t p = m.p;
+      const uint32_t c = (uint32_t)((1ull << 63) - p);
+      uint64_t r, s;
+      gi_mul_pm(r, s, a0, b0, p, c);
+      c21[i] = make_ulonglong2(r, s);
+      gi_mul_pm(r, s, a1, b1, p, c);
+      c23[i] = make_ulonglong2(r, s);
+      ProductSum<false> re, im;
+      re.mac(a0.x, b1.x);
+      re.mac(a0.y, p - b1.y);
+      re.mac(a1.x, b0.x);
+      re.mac(a1.y, p - b0.y);
+      im.mac(a0.x, b1.y);
+      im.mac(a0.y, b1.x);
+      im.mac(a1.x, b0.y);
+      im.mac(a1.y, b0.x);
+      c22[i] = make_ulonglong2(canon(re.fold(c), c, p), canon(im.fold(c), c, p));
+      return;
+    }
     uint64_t r1, i1, r2, i2, r3, i3, r4, i4;
     gi_mul(r1, i1, a0.x, a0.y, b0.x, b0.y, m);
     gi_mul(r2, i2, a0.x, a0.y, b1.x, b1.y, m);
@@ -176,17 +210,17 @@ template <class Load>
 __device__ __forceinline__ u2 dot_elem(int n, const ModConst& m, Load load) {
   uint64_t sr = 0, si = 0;
   if (m.pm) {
-    uint64_t l1 = 0, h1 = 0, t1 = 0, l2 = 0, h2 = 0, t2 = 0, l3 = 0, h3 = 0, t3 = 0;
+    const uint32_t c = (uint32_t)((1ull << 63) - m.p);
+    ProductSum<true> s1, s2, s3;
 #pragma unroll 4
     for (int t = 0; t < n; ++t) {
       u2 x, y;
       load(t, x, y);
-      mac192(l1, h1, t1, x.x, y.x);
-      mac192(l2, h2, t2, x.y, y.y);
-      mac192(l3, h3, t3, x.x + x.y, y.x + y.y);
+      s1.mac(x.x, y.x);
+      s2.mac(x.y, y.y);
+      s3.mac(x.x + x.y, y.x + y.y);
     }
-    const uint64_t p1 = red192(l1, h1, t1, m.p, m.r1, m.r2), p2 = red192(l2, h2, t2, m.p, m.r1, m.r2),
-                   p3 = red192(l3, h3, t3, m.p, m.r1, m.r2);
+    const uint64_t p1 = canon(s1.fold(c), c, m.p), p2 = canon(s2.fold(c), c, m.p), p3 = canon(s3.fold(c), c, m.p);
     sr = sub_mod(p1, p2, m.p);
     si = sub_mod(sub_mod(p3, p1, m.p), p2, m.p);
   } else {
@@ -254,12 +288,13 @@ int pw_double_add(const Engine& e, void* c1, const void* a1, const void* b1, voi
                   const void* b2, int base, cudaStream_t st) {
   return launch_ew(e, DoubleAddF{U2(c1), U2(c2), CU2(a1), CU2(b1), CU2(a2), CU2(b2)}, base, st);
 }
-int pw_mul(const Engine& e, void* c, const void* a, const void* b, int base, cudaStream_t st, int npolys) {
-  return launch_ew(e, MulF{U2(c), CU2(a), CU2(b)}, base, st, npolys);
+int pw_mul(const Engine& e, void* c, const void* a, const void* b, int base, cudaStream_t st, int npolys,
+           bool any_rows) {
+  return launch_ew(e, MulF{U2(c), CU2(a), CU2(b)}, base, st, npolys, nullptr, any_rows);
 }
 int pw_mul_list(const Engine& e, void* c, const void* a, const void* b, const int* rid_list, int nlist,
-                cudaStream_t st) {
-  return launch_ew(e, MulF{U2(c), CU2(a), CU2(b)}, 0, st, nlist, rid_list);
+                cudaStream_t st, bool any_rows) {
+  return launch_ew(e, MulF{U2(c), CU2(a), CU2(b)}, 0, st, nlist, rid_list, any_rows);
 }
 int pw_mul_u64(const Engine& e, void* c, const void* a, const uint64_t* b, int base, cudaStream_t st) {
   return launch_ew(e, MulU64F{U2(c), CU2(a), b}, base, st);
@@ -325,8 +360,9 @@ int pw_dot_batch(const Engine& e, void* c, const void* a, const void* b, int n, 
   return check_launch("dot_batch");
 }
 int pw_dr2(const Engine& e, void* c21, void* c22, void* c23, const void* c01, const void* c02, const void* c11,
-           const void* c12, int base, cudaStream_t st, int npolys) {
-  return launch_ew(e, Dr2F{U2(c21), U2(c22), U2(c23), CU2(c01), CU2(c02), CU2(c11), CU2(c12)}, base, st, npolys);
+           const void* c12, int base, cudaStream_t st, int npolys, bool any_rows) {
+  return launch_ew(e, Dr2F{U2(c21), U2(c22), U2(c23), CU2(c01), CU2(c02), CU2(c11), CU2(c12)}, base, st, npolys, nullptr,
+                   any_rows);
 }
 int pw_negate(const Engine& e, void* b, const void* a, int base, cudaStream_t st) {
   return launch_ew(e, NegF{U2(b), CU2(a)}, base, st);

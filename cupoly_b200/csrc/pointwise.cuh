@@ -10,10 +10,12 @@ int pw_add(const Engine& e, void* c, const void* a, const void* b, int base, cud
 int pw_sub(const Engine& e, void* c, const void* a, const void* b, int base, cudaStream_t st);
 int pw_double_add(const Engine& e, void* c1, const void* a1, const void* b1, void* c2, const void* a2,
                   const void* b2, int base, cudaStream_t st);
-int pw_mul(const Engine& e, void* c, const void* a, const void* b, int base, cudaStream_t st, int npolys = 1);
+// any_rows: batches of any number of rows (the plain calls refuse some above 65535)
+int pw_mul(const Engine& e, void* c, const void* a, const void* b, int base, cudaStream_t st, int npolys = 1,
+           bool any_rows = false);
 int pw_mul_u64(const Engine& e, void* c, const void* a, const uint64_t* b, int base, cudaStream_t st);
 int pw_mul_list(const Engine& e, void* c, const void* a, const void* b, const int* rid_list, int nlist,
-                cudaStream_t st);
+                cudaStream_t st, bool any_rows = false);
 int pw_muladd(const Engine& e, void* d, const void* a, const void* b, const void* c, int base, cudaStream_t st);
 // Operand pairs per dot-product launch; longer sums take several launches.
 constexpr int kDotTerms = 64;
@@ -22,7 +24,7 @@ int pw_dot(const Engine& e, void* c, const void* const* a, const void* const* b,
 int pw_dot_batch(const Engine& e, void* c, const void* a, const void* b, int n, int npolys, bool b_shared, int base,
                  cudaStream_t st);
 int pw_dr2(const Engine& e, void* c21, void* c22, void* c23, const void* c01, const void* c02, const void* c11,
-           const void* c12, int base, cudaStream_t st, int npolys = 1);
+           const void* c12, int base, cudaStream_t st, int npolys = 1, bool any_rows = false);
 int pw_negate(const Engine& e, void* b, const void* a, int base, cudaStream_t st);
 int pw_op_by_int(const Engine& e, void* b, const void* a, int base, uint64_t x, int op, cudaStream_t st);
 int pw_double_op_by_int(const Engine& e, void* b1, const void* a1, void* b2, const void* a2, int base, uint64_t x1,
