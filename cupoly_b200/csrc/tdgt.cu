@@ -20,9 +20,13 @@
 // is part of the first twiddle), a twiddle is two products, and the first and last pass's
 // matrices (32 x 32 residues) convert between the forms.
 //
-// Measured on B200, forward / inverse of 402 MB of residues (3072 at N = 4096): N = 1024 162 /
-// 182 us, 2048 164 / 174, 4096 172 / 195, 8192 219 / 223 us; the CUDA-core kernels 251 / 260,
-// 267 / 273, 316 / 308, 332 / 351 us.
+// Measured on B200, forward / inverse of 201 MB of residues (3072 at N = 4096, 62 us of traffic):
+// N = 1024 160 / 163 us, 2048 160 / 152, 4096 172 / 181, 8192 221 / 214 us; the CUDA-core kernels
+// 260 / 263, 267 / 274, 318 / 314, 332 / 345 us.  What bounds it: a unit's passes depend on each
+// other, so its products (57 us at N = 4096) and its arithmetic (82 us of issue slots) overlap only
+// across the two tiles of a pass.  Two units in flight on pairs of CTAs (cta_group::2, half of the
+// matrices in each) were slower, 219 / 265 us: the hand-over between the CTAs on every pass costs
+// more than the overlap gives.
 //
 // One persistent CTA per SM walks units of 4096 elements (8192 for N = 8192; 4096 / N
 // residues of one prime for the smaller sizes) ordered by prime, so the matrices stay in
@@ -101,6 +105,12 @@ __device__ __forceinline__ uint64_t mul_lazy(uint64_t a, ulonglong2 w, const Red
   return mad_wide(k, C, pack64(l0, l1));
 }
 
+// A twiddle pair (32 bytes, aligned) in one load: half the load instructions between the
+// reductions (with the pairs loaded three steps ahead, inverse at N = 4096: 195 us before, 181 so).
+__device__ __forceinline__ void ldg32(ulonglong2 (&w)[2], const ulonglong2* p) {
+  asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(w[0].x), "=l"(w[0].y), "=l"(w[1].x), "=l"(w[1].y) : "l"(p));
+}
+
 __device__ __forceinline__ void sts8(uint32_t a, uint64_t v) {
   asm volatile("st.shared.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
 }
@@ -113,9 +123,9 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // One residue (element block) of the launch.
 struct Item {
-  size_t off;   // element offset of the output (and of the input of modes 0 and 3)
-  size_t pair;  // gather / tensor modes: offset inside each operand
-  int j;        // operand (gather) or tensor output
+  size_t off;   // element offset of the output (and of the input of mode 0)
+  size_t pair;  // gather mode: offset inside the operand
+  int j;        // gather mode: operand
   int q, blk;   // polynomial (list: row) and element block in it
 };
 
@@ -124,16 +134,11 @@ __device__ __forceinline__ Item item_of(const TArgs& A, unsigned r, unsigned it)
   constexpr int LOGN = Cfg<M>::LOGN;
   Item I;
   const unsigned h = it & ((1u << A.S) - 1);
-  unsigned q = it >> A.S;
+  const unsigned q = it >> A.S;
   const size_t inner = ((size_t)r << (LOGN + A.S)) + ((size_t)h << LOGN);
   I.j = 0;
   I.pair = 0;
-  if (INV && A.isrc.mode == 1) {  // c0, c1, c2 of one pair in adjacent items: the operands stay in L2
-    I.j = (int)(q % 3);
-    const unsigned pr = q / 3;
-    q = I.j * A.isrc.npairs + pr;
-    I.pair = pr * A.poly_stride + inner;
-  } else if (INV && A.isrc.mode == 2) {
+  if (INV && A.isrc.mode == 2) {
     I.j = (int)(q / A.isrc.npairs);
     I.pair = (q % A.isrc.npairs) * A.poly_stride + inner;
   }
@@ -141,6 +146,293 @@ __device__ __forceinline__ Item item_of(const TArgs& A, unsigned r, unsigned it)
   I.q = (int)q;
   I.blk = (int)((r << A.S) + h);
   return I;
+}
+
+// The reductions between the products, by 8 warps over a tile of 128 rows: thread (row, wh) takes
+// 8 elements (u, v), half wh of the row's outputs.  `wait` waits for the tile's product, `read`
+// tells that its columns are in registers.
+template <int M, bool INV>
+struct Epilogue {
+  using C = Cfg<M>;
+  static constexpr int N2 = C::N2, NM = C::NM;
+  static constexpr int kAhead = 3;  // steps between a twiddle's load and its use
+  uint32_t sdat;  // the unit's shared memory
+  uint32_t tl;    // the buffer's tensor memory, this warp's lanes
+  int warp, lane, row, wh;
+  Red R_;
+
+  // 8 steps of 16 columns: two sums a step by `sums`, then `body` on them one step later, so
+  // that the two dependent chains of a step overlap the next step's; and the columns after
+  // those are on their way meanwhile.
+  template <class Read, class Ld, class Sums, class Body>
+  __device__ __forceinline__ void steps(Read read, Ld ld, Sums sums, Body body) const {
+    uint32_t c[2][16];
+    uint64_t x[2], y[2];
+    ld(0, c[0]);
+#pragma unroll
+    for (int s = 0; s < 9; ++s) {
+      if (s < 8) {
+        tmem_ld_wait(c[s & 1]);
+        if (s == 7) read();  // the buffer's columns are in registers
+        if (s < 7) ld(s + 1, c[(s + 1) & 1]);
+        sums(c[s & 1], x[s & 1], y[s & 1], R_);
+      }
+      if (s > 0) body(s - 1, x[(s - 1) & 1], y[(s - 1) & 1]);
+    }
+  }
+  static __device__ __forceinline__ void sum2(const uint32_t* c, uint64_t& x, uint64_t& y, const Red& r) {
+    x = col_sum(c, r);
+    y = col_sum(c + 8, r);
+  }
+
+  // First pass of tile t: columns -> twiddled -> the middle pass's operand.
+  template <class Wait, class Read>
+  __device__ __forceinline__ void first(int t, const ulonglong2* T1, const ulonglong2* T2, Wait wait, Read read) const {
+    auto ld_seq = [&](int s, uint32_t(&c)[16]) { tmem_ld16(c, tl + 128 * wh + 16 * s); };
+    if (!INV) {
+      const int nmi = M == 2 ? (row >> 4) & 3 : row >> 4, nl = row & 15;
+      const int n2 = M >= 4 ? 128 * t + row : (M == 3 ? row : row & 63);
+      const ulonglong2* Tw = T1 + 2 * (8 * wh * N2 + n2);
+      ulonglong2 w[kAhead + 1][2];
+      auto ldw = [&](int s) {
+        ldg32(w[s & kAhead], Tw + 2 * s * N2);
+      };
+#pragma unroll
+      for (int s = 0; s < kAhead; ++s) ldw(s);
+      wait();
+      const int R0 = (M == 2 ? (row >> 6) * 512 : 0) + wh * 256 + nl;  // q1 = 8 wh, u
+      constexpr int RB = M == 2 ? 32 : 64;
+      const uint32_t base = sdat + t * 32768 + R0 * RB + (nmi & 1) * 8 +
+                            (((nmi >> 1) ^ (M == 2 ? (R0 >> 2) & 1 : (R0 >> 1) & 3)) << 4);
+      steps(read, ld_seq, sum2, [&](int s, uint64_t x, uint64_t y) {
+        if (s + kAhead < 8) ldw(s + kAhead);
+        sts8(base + s * 16 * RB, mul_lazy(x, w[s & kAhead][0], R_));
+        sts8(base + (128 + s * 16) * RB, mul_lazy(y, w[s & kAhead][1], R_));
+      });
+    } else {
+      const int qm = row & (NM - 1), q1l = M == 2 ? (row >> 2) & 15 : row >> M;
+      // digit nl = 8 wh + j: every layout xors bits of nl below the first that depends on wh
+      uint32_t base;
+      int ch;  // swizzled chunk before the xor with bits of nl
+      if (M == 4) {
+        base = t * 32768 + (q1l * 16 + 8 * wh) * 128 + (qm & 1) * 8;
+        ch = qm >> 1;
+      } else if (M == 5) {
+        base = t * 32768 + (qm >> 4) * 16384 + (q1l * 16 + 8 * wh) * 128 + (qm & 1) * 8;
+        ch = (qm & 15) >> 1;
+      } else if (M == 3) {
+        base = t * 32768 + ((q1l >> 3) * 256 + (q1l & 7) * 16 + 8 * wh) * 64 + (qm & 1) * 8;
+        ch = qm >> 1;
+      } else {
+        base = t * 32768 + ((row >> 6) * 512 + (q1l >> 3) * 256 + (q1l & 7) * 16 + 8 * wh) * 32 + (qm & 1) * 8;
+        ch = qm >> 1;
+      }
+      base += sdat;
+      constexpr int RB = M >= 4 ? 128 : (M == 3 ? 64 : 32);
+      constexpr int UV = M == 4 ? 16384 : (M == 5 ? 64 * 128 : 128 * RB);
+      const ulonglong2* Tw = T2 + 8 * wh * NM + qm;
+      wait();
+      steps(read, ld_seq, sum2, [&](int j, uint64_t x, uint64_t y) {
+        const ulonglong2 w = __ldg(Tw + j * NM);
+        const int sw = M >= 4 ? j : (M == 3 ? (j >> 1) & 3 : (j >> 2) & 1);
+        const uint32_t a = base + j * RB + ((ch ^ sw) << 4);
+        sts8(a, mul_lazy(x, w, R_));
+        sts8(a + UV, mul_lazy(y, w, R_));
+      });
+    }
+  }
+
+  // Middle pass of tile t: N = 4096 forward: t = half h; N = 8192 forward: t = 2 h + s.
+  template <class Wait, class Read>
+  __device__ __forceinline__ void middle(int t, const ulonglong2* T1, const ulonglong2* T2, Wait wait, Read read) const {
+    auto ld_seq = [&](int s, uint32_t(&c)[16]) { tmem_ld16(c, tl + 128 * wh + 16 * s); };
+    // u and v of output s of this half
+    auto ld_uv = [&](int s, uint32_t(&c)[16]) {
+      if (M >= 4)
+        tmem_ld8x2(c, tl + 64 * wh + 8 * s, tl + 128 + 64 * wh + 8 * s);
+      else if (M == 3)
+        tmem_ld8x2(c, tl + 128 * wh + 8 * s, tl + 128 * wh + 64 + 8 * s);
+      else
+        tmem_ld8x2(c, tl + (2 * wh + (s >> 2)) * 64 + 8 * (s & 3), tl + (2 * wh + (s >> 2)) * 64 + 32 + 8 * (s & 3));
+    };
+    const int q1l = row >> 4, nl = row & 15;
+    if (!INV) {
+      const int o0 = M == 5 ? 16 * (t & 1) + 8 * wh : (M == 4 ? 8 * wh : 0);  // first digit qm
+      const ulonglong2* Tw = T2 + o0 * 16 + nl;
+      wait();
+      steps(read, ld_uv, sum2, [&](int s, uint64_t x, uint64_t y) {
+        const int oj = M == 2 ? s & 3 : s;
+        const ulonglong2 w = __ldg(Tw + oj * 16);
+        const int qm = o0 + oj, pn = nl >> 3;
+        int r3;
+        uint32_t a;
+        if (M == 5) {
+          r3 = q1l * 32 + qm;
+          a = (pn * 2 + (r3 >> 7)) * 32768 + (t >> 1) * 16384 + (r3 & 127) * 128;
+        } else if (M == 4) {
+          r3 = q1l * 16 + qm;
+          a = pn * 32768 + t * 16384 + r3 * 128;
+        } else if (M == 3) {
+          r3 = (wh * 8 + q1l) * 8 + qm;
+          a = t * 32768 + pn * 16384 + r3 * 128;
+        } else {
+          r3 = wh * 64 + ((s >> 2) * 8 + q1l) * 4 + qm;
+          a = t * 32768 + pn * 16384 + r3 * 128;
+        }
+        sts16(sdat + a + (((nl & 7) ^ (r3 & 7)) << 4), mul_lazy(x, w, R_), mul_lazy(y, w, R_));
+      });
+    } else if (M != 5) {
+      // M == 2: row tiles 2 wh (q1 = q1l) and 2 wh + 1 (q1 = 8 + q1l) of residue wh, 4 outputs each
+      const int q1 = M == 4 ? 8 * t + q1l : (M == 3 ? wh * 8 + q1l : q1l);
+      const int o0 = M == 4 ? 8 * wh : 0;  // first digit nm
+      const ulonglong2* Tw = T1 + 2 * (q1 * N2 + 16 * o0 + nl);
+      auto tw_off = [&](int s) { return M == 2 ? 2 * ((s >> 2) * 8 * N2 + 16 * (s & 3)) : 32 * s; };
+      ulonglong2 w[kAhead + 1][2];
+      auto ldw = [&](int s) {
+        ldg32(w[s & kAhead], Tw + tw_off(s));
+      };
+#pragma unroll
+      for (int s = 0; s < kAhead; ++s) ldw(s);
+      wait();
+      const int n2 = 16 * o0 + nl;
+      const uint32_t a = sdat + t * 32768 +
+                         (M == 4 ? n2 * 128 : (M == 3 ? wh * 16384 + n2 * 128 : (wh * 64 + n2) * 128)) +
+                         ((q1l ^ (nl & 7)) << 4);
+      steps(read, ld_uv, sum2, [&](int s, uint64_t x, uint64_t y) {
+        if (s + kAhead < 8) ldw(s + kAhead);
+        sts16(a + (M == 2 ? (s & 3) * 2048 + (s >> 2) * 16384 : s * 2048), mul_lazy(x, w[s & kAhead][0], R_),
+              mul_lazy(y, w[s & kAhead][1], R_));
+      });
+    } else {  // N = 8192: rows of u (lanes 0 .. 63) or of v; 16 outputs each
+      const int uv = row >> 6, q1 = 4 * t + ((row >> 4) & 3), o0 = 16 * wh;
+      const ulonglong2* Tw = T1 + 2 * (q1 * N2 + 16 * o0 + nl) + uv;
+      ulonglong2 w[kAhead + 1][2];
+      auto ldw = [&](int s) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) w[s & kAhead][i] = __ldg(Tw + 32 * (2 * s + i));
+      };
+#pragma unroll
+      for (int s = 0; s < kAhead; ++s) ldw(s);
+      wait();
+      const uint32_t a = sdat + (t >> 1) * 65536 + (16 * o0 + nl) * 128 + (((q1 & 7) ^ (nl & 7)) << 4) + uv * 8;
+      steps(read, ld_seq, sum2, [&](int s, uint64_t x, uint64_t y) {
+        if (s + kAhead < 8) ldw(s + kAhead);
+        sts8(a + 2 * s * 2048, mul_lazy(x, w[s & kAhead][0], R_));
+        sts8(a + (2 * s + 1) * 2048, mul_lazy(y, w[s & kAhead][1], R_));
+      });
+    }
+  }
+
+  // Last pass of tile t: canonical results to global memory; out(g) is item g of the unit or nullptr.
+  template <class Out, class Read>
+  __device__ __forceinline__ void last(int t, Out out, Read read) const {
+    auto ld_seq = [&](int s, uint32_t(&c)[16]) { tmem_ld16(c, tl + 128 * wh + 16 * s); };
+    if (INV) {
+      const int g = M >= 4 ? 0 : (M == 3 ? t : 2 * t + (row >> 6));
+      const int n2 = M >= 4 ? 128 * t + row : (M == 3 ? row : row & 63);
+      ulonglong2* x0 = out(g);
+      const bool live = x0 != nullptr;
+      ulonglong2* x = x0 + 8 * wh * N2 + n2;
+      steps(read, ld_seq, sum2, [&](int s, uint64_t a, uint64_t b) {
+        if (live) x[s * N2] = make_ulonglong2(red2p(a, R_.p), red2p(b, R_.p));
+      });
+    } else {
+      // A row's results are contiguous: four neighbouring lanes take four elements of a row
+      // (64 bytes a store), so that a store instruction touches 8 lines and not 32.
+      const int rw = (warp & 3) * 32;  // rows of this warp; M == 2: all of one residue
+      const int g = M >= 4 ? 0 : (M == 3 ? t : 2 * t + (rw >> 6));
+      const int r0 = M >= 4 ? 128 * t + rw : (M == 3 ? rw : rw & 63);
+      ulonglong2* x0 = out(g);
+      const bool live = x0 != nullptr;
+      ulonglong2* x = x0 + (r0 + (lane >> 2)) * 16 + 8 * wh + (lane & 3);
+      uint64_t z0 = 0, z1 = 0;
+      // step: 16-lane half s >> 2, group of 4 elements (s >> 1) & 1, component s & 1
+      steps(read, [&](int s, uint32_t(&c)[16]) {
+        tmem_ld_quad(c, tl + ((uint32_t)((s >> 2) * 16) << 16) + 128 * wh + 32 * (s & 3));
+      }, [](const uint32_t* c, uint64_t& x, uint64_t& y, const Red& R_) {
+        x = col_sum(c[0], c[1], c[4], c[5], c[8], c[9], c[12], c[13], R_);
+        y = col_sum(c[2], c[3], c[6], c[7], c[10], c[11], c[14], c[15], R_);
+      }, [&](int s, uint64_t a, uint64_t b) {
+        a = red2p(a, R_.p);
+        b = red2p(b, R_.p);
+        if (s & 1) {
+          ulonglong2* y = x + (s >> 2) * 256 + 4 * ((s >> 1) & 1);
+          if (live) {
+            y[0] = make_ulonglong2(z0, a);
+            y[128] = make_ulonglong2(z1, b);
+          }
+        } else {
+          z0 = a;
+          z1 = b;
+        }
+      });
+    }
+  }
+};
+
+// Inverse: tiles t0, t0 + dt, ... of a unit's operand into shared memory by 256 threads (gtid),
+// swizzled rows of 16 elements; item(g) is item g < count of the unit.
+template <int M, class ItemOf>
+__device__ __forceinline__ void load_inverse(const TArgs& A, uint32_t sdat, int gtid, int t0, int dt, int count,
+                                             ItemOf item) {
+#pragma unroll 1
+  for (int t = t0; t < Cfg<M>::TILES; t += dt) {
+#pragma unroll 1
+    for (int g0 = 0; g0 < (M == 2 ? 2 : 1); ++g0) {
+      const int g = M == 2 ? 2 * t + g0 : (M == 3 ? t : 0);
+      if (g >= count) continue;
+      const Item I = item(g);
+      constexpr int E = M == 2 ? 1024 : 2048;  // elements of this item in this tile
+      const int eo = M >= 4 ? t * 2048 : 0;    // their first element in the item
+      const int er0 = (gtid >> 4) + (M == 2 ? g0 * 64 : 0), ql = gtid & 15;
+      // rows er0, er0 + 16, ...: the swizzle term does not change
+      const uint32_t dst0 = sdat + t * 32768 + (ql >> 3) * 16384 + er0 * 128 + (((ql & 7) ^ (er0 & 7)) << 4);
+      const ulonglong2* src =
+          (A.isrc.mode == 0 ? A.isrc.p[0] + I.off : inv_src_ptr(A.isrc, I.j) + I.pair) + eo + gtid;
+#pragma unroll
+      for (int i = 0; i < E / 256; ++i) cp_async16(dst0 + i * 2048, src + i * 256);
+    }
+  }
+}
+
+// Orders the rows of a work list by prime (each CTA for itself: no scratch memory, no second
+// launch): rows cnt[r] .. cnt[r + 1] of `order` have prime r, and units of at most GR rows start
+// at ustart[r].  Returns the number of units.
+template <int GR>
+__device__ __forceinline__ unsigned order_rows(const TArgs& A, unsigned* s_cnt, unsigned* s_ustart, uint16_t* s_order,
+                                               int warp, int lane, int tid, int threads) {
+  for (int i = tid; i <= kMaxResidues; i += threads) s_cnt[i] = 0;
+  __syncthreads();
+  for (int i = tid; i < A.nlist; i += threads) {
+    const unsigned r = (unsigned)A.rid_list[i];
+    if (r < (unsigned)A.nprimes) atomicAdd(&s_cnt[r + 1], 1u);  // a row of no prime of the engine is left out
+  }
+  __syncthreads();
+  if (tid == 0) {
+    unsigned u = 0, c = 0;
+    for (int r = 0; r < kMaxResidues; ++r) {
+      const unsigned n = s_cnt[r + 1];
+      s_ustart[r] = u;
+      u += (n + GR - 1) / GR;
+      s_cnt[r] = c;  // first row of prime r in the order
+      c += n;
+    }
+    s_ustart[kMaxResidues] = u;
+    s_cnt[kMaxResidues] = c;
+  }
+  __syncthreads();
+  // stable order without atomics: a warp takes every (threads / 32)-th prime
+  for (int r = warp; r < kMaxResidues; r += (threads >> 5)) {
+    unsigned at = s_cnt[r];
+    const unsigned end = s_cnt[r + 1];
+    for (int b = 0; b < A.nlist && at < end; b += 32) {
+      const bool mine = b + lane < A.nlist && A.rid_list[b + lane] == r;
+      const unsigned m = __ballot_sync(0xFFFFFFFFu, mine);
+      if (mine) s_order[at + __popc(m & ((1u << lane) - 1))] = (uint16_t)(b + lane);
+      at += __popc(m);
+    }
+  }
+  return s_ustart[kMaxResidues];
 }
 
 // `fmap` (forward): the input as a tensor of 64-bit words, {2 N2, 16 x blocks, polynomials}; for
@@ -177,40 +469,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == kEpiWarps) tmem_alloc(smem_u32(&s_slot), 512);
   const bool list = A.rid_list != nullptr;
   unsigned nunits = A.nunits;
-  if (list) {  // order the rows by prime (each CTA for itself: no scratch memory, no second launch)
-    for (int i = tid; i <= kMaxResidues; i += kThreads) s_cnt[i] = 0;
-    __syncthreads();
-    for (int i = tid; i < A.nlist; i += kThreads) {
-      const unsigned r = (unsigned)A.rid_list[i];
-      if (r < (unsigned)A.nprimes) atomicAdd(&s_cnt[r + 1], 1u);  // a row of no prime of the engine is left out
-    }
-    __syncthreads();
-    if (tid == 0) {
-      unsigned u = 0, c = 0;
-      for (int r = 0; r < kMaxResidues; ++r) {
-        const unsigned n = s_cnt[r + 1];
-        s_ustart[r] = u;
-        u += (n + G - 1) / G;
-        s_cnt[r] = c;  // first row of prime r in the order
-        c += n;
-      }
-      s_ustart[kMaxResidues] = u;
-      s_cnt[kMaxResidues] = c;
-    }
-    __syncthreads();
-    // stable order without atomics: warp w takes the primes w, w + 17, ...
-    for (int r = warp; r < kMaxResidues; r += kEpiWarps + 1) {
-      unsigned at = s_cnt[r];
-      const unsigned end = s_cnt[r + 1];
-      for (int b = 0; b < A.nlist && at < end; b += 32) {
-        const bool mine = b + lane < A.nlist && A.rid_list[b + lane] == r;
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, mine);
-        if (mine) s_order[at + __popc(m & ((1u << lane) - 1))] = (uint16_t)(b + lane);
-        at += __popc(m);
-      }
-    }
-    nunits = s_ustart[kMaxResidues];
-  }
+  if (list) nunits = order_rows<G>(A, s_cnt, s_ustart, s_order, warp, lane, tid, kThreads);
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
@@ -375,16 +634,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           constexpr uint32_t bytes = C::N * 16;
           if (!INV) {
             prefetch_l2(A.fsrc + I.off, bytes);
-          } else if (A.isrc.mode == 0 || A.isrc.mode == 3) {
-            prefetch_l2(A.isrc.p[0] + I.off, bytes);
-            if (A.isrc.mode == 3) prefetch_l2(A.isrc.p[1] + I.off, bytes);
-          } else if (A.isrc.mode == 2) {
-            prefetch_l2(inv_src_ptr(A.isrc, I.j) + I.pair, bytes);
           } else {
-            if (I.j != 2) prefetch_l2(A.isrc.p[0] + I.pair, bytes);
-            if (I.j != 0) prefetch_l2(A.isrc.p[1] + I.pair, bytes);
-            if (I.j != 2) prefetch_l2(A.isrc.p[2] + I.pair, bytes);
-            if (I.j != 0) prefetch_l2(A.isrc.p[3] + I.pair, bytes);
+            prefetch_l2(A.isrc.mode == 0 ? A.isrc.p[0] + I.off : inv_src_ptr(A.isrc, I.j) + I.pair, bytes);
           }
         }
         if (list) cur_r = r;  // unit_of walks forward only
@@ -502,10 +753,17 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncwarp();
   } else {
     // Two groups of 8 warps: group d reduces the products of buffer d, so one group's waits
-    // and fences overlap the other's arithmetic.  A warp reads its 32 lanes; the two halves
-    // `wh` of a group share the columns, 8 elements (u, v) a thread and tile in 4 steps of 2.
-    const int d = warp >> 3, wh = (warp >> 2) & 1, row = (warp & 3) * 32 + lane;
-    const uint32_t tl = tmem + 256 * d + ((uint32_t)((warp & 3) * 32) << 16);
+    // and fences overlap the other's arithmetic.
+    const int d = warp >> 3, gtid = tid & 255;
+    uint32_t k8 = 256;  // see Red
+    asm volatile("" : "+r"(k8));
+    Epilogue<M, INV> ep;
+    ep.sdat = sdat;
+    ep.warp = warp;
+    ep.lane = lane;
+    ep.row = (warp & 3) * 32 + lane;
+    ep.wh = (warp >> 2) & 1;
+    ep.tl = tmem + 256 * d + ((uint32_t)((warp & 3) * 32) << 16);
     uint32_t pd = 0;
     auto waitD = [&]() {
       mbar_wait(bD + 8 * d, pd & 1, &s_fail);
@@ -529,56 +787,12 @@ __global__ void __launch_bounds__(kThreads, 1)
       fence_async_smem();
       doneE();
     };
-    // inverse: the operand tiles of this group, swizzled rows of 16 elements
-    const int gtid = tid & 255;
-    auto load_inv = [&](unsigned u) {
+    auto none = []() {};
+    auto load_unit = [&](unsigned u) {
       int r, count;
       unsigned first;
       unit_of(u, r, first, count);
-      const ModConst m = A.mc[rid_of(r)];
-#pragma unroll 1
-      for (int t = d; t < TILES; t += 2) {
-#pragma unroll 1
-        for (int g0 = 0; g0 < (M == 2 ? 2 : 1); ++g0) {
-          const int g = M == 2 ? 2 * t + g0 : (M == 3 ? t : 0);
-          if (g >= count) continue;
-          const Item I = item_at(r, first + g);
-          constexpr int E = M == 2 ? 1024 : 2048;  // elements of this item in this tile
-          const int eo = M >= 4 ? t * 2048 : 0;    // their first element in the item
-          const int er0 = (gtid >> 4) + (M == 2 ? g0 * 64 : 0), ql = gtid & 15;
-          // rows er0, er0 + 16, ...: the swizzle term does not change
-          const uint32_t dst0 = sdat + t * 32768 + (ql >> 3) * 16384 + er0 * 128 + (((ql & 7) ^ (er0 & 7)) << 4);
-          const int mode = A.isrc.mode;
-          if (mode == 0 || mode == 2) {
-            const ulonglong2* src = (mode == 0 ? A.isrc.p[0] + I.off : inv_src_ptr(A.isrc, I.j) + I.pair) + eo + gtid;
-#pragma unroll
-            for (int i = 0; i < E / 256; ++i) cp_async16(dst0 + i * 2048, src + i * 256);
-          } else if (mode == 3) {
-            const ulonglong2 *pa = A.isrc.p[0] + I.off + eo + gtid, *pb = A.isrc.p[1] + I.off + eo + gtid;
-#pragma unroll 4
-            for (int i = 0; i < E / 256; ++i) {
-              const ulonglong2 a = pa[i * 256], b = pb[i * 256];
-              uint64_t cr, ci;
-              gi_mul(cr, ci, a.x, a.y, b.x, b.y, m);
-              sts16(dst0 + i * 2048, cr, ci);
-            }
-          } else {
-            auto all = [&](auto out) {  // the output index as a constant: one loop per output
-#pragma unroll 2
-              for (int i = 0; i < E / 256; ++i) {
-                const ulonglong2 z = tensor_load(A.isrc, decltype(out)::value, I.pair + eo + gtid + i * 256, m);
-                sts16(dst0 + i * 2048, z.x, z.y);
-              }
-            };
-            if (I.j == 0)
-              all(std::integral_constant<int, 0>{});
-            else if (I.j == 2)
-              all(std::integral_constant<int, 2>{});
-            else
-              all(std::integral_constant<int, 1>{});
-          }
-        }
-      }
+      load_inverse<M>(A, sdat, gtid, d, 2, count, [&](int g) { return item_at(r, first + g); });
     };
     auto load_done = [&]() {
       cp_async_wait();
@@ -588,186 +802,32 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int t = d; t < TILES; t += 2) mbar_arrive(bA + 8 * t);
     };
     if (INV && u0 < u1) {
-      load_inv(u0);
+      load_unit(u0);
       load_done();
     }
-    uint32_t k8 = 256;  // see Red
-    asm volatile("" : "+r"(k8));
-    // 8 steps of 16 columns: two sums a step by `sums`, then `body` on them one step later, so
-    // that the two dependent chains of a step overlap the next step's; and the columns after
-    // those are on their way meanwhile.
-    auto steps = [&](const Red& R_, auto ld, auto sums, auto body) {
-      uint32_t c[2][16];
-      uint64_t x[2], y[2];
-      ld(0, c[0]);
-#pragma unroll
-      for (int s = 0; s < 9; ++s) {
-        if (s < 8) {
-          tmem_ld_wait(c[s & 1]);
-          if (s < 7) ld(s + 1, c[(s + 1) & 1]);
-          sums(c[s & 1], x[s & 1], y[s & 1], R_);
-        }
-        if (s > 0) body(s - 1, x[(s - 1) & 1], y[(s - 1) & 1]);
-      }
-    };
-    auto sum2 = [](const uint32_t* c, uint64_t& x, uint64_t& y, const Red& R_) {
-      x = col_sum(c, R_);
-      y = col_sum(c + 8, R_);
-    };
-    auto ld_seq = [&](int s, uint32_t(&c)[16]) { tmem_ld16(c, tl + 128 * wh + 16 * s); };
-    // u and v of output s of this half (middle pass)
-    auto ld_uv = [&](int s, uint32_t(&c)[16]) {
-      if (M >= 4)
-        tmem_ld8x2(c, tl + 64 * wh + 8 * s, tl + 128 + 64 * wh + 8 * s);
-      else if (M == 3)
-        tmem_ld8x2(c, tl + 128 * wh + 8 * s, tl + 128 * wh + 64 + 8 * s);
-      else
-        tmem_ld8x2(c, tl + (2 * wh + (s >> 2)) * 64 + 8 * (s & 3), tl + (2 * wh + (s >> 2)) * 64 + 32 + 8 * (s & 3));
-    };
-    constexpr int kAhead = 3;  // steps between a twiddle's load and its use
     for (unsigned u = u0; u < u1; ++u) {
       int r, count;
       unsigned first;
       unit_of(u, r, first, count);
       const int rid = rid_of(r);
       const uint64_t p = A.mc[rid].p;
-      const Red R_{p, (uint32_t)((1ull << 63) - p), k8, k8 << 8};
+      ep.R_ = Red{p, (uint32_t)((1ull << 63) - p), k8, k8 << 8};
       const uint8_t* tab = A.tab + (size_t)rid * A.L.stride;
       const ulonglong2* T1 = reinterpret_cast<const ulonglong2*>(tab + (INV ? A.L.i_t1 : A.L.f_t1));
       const ulonglong2* T2 = reinterpret_cast<const ulonglong2*>(tab + (INV ? A.L.i_t2 : A.L.f_t2));
-      // ---- pass 1 ----
 #pragma unroll 1
       for (int t = d; t < TILES; t += 2) {
-        if (!INV) {
-          const int nmi = M == 2 ? (row >> 4) & 3 : row >> 4, nl = row & 15;
-          const int n2 = M >= 4 ? 128 * t + row : (M == 3 ? row : row & 63);
-          const ulonglong2* Tw = T1 + 2 * (8 * wh * N2 + n2);
-          ulonglong2 w[kAhead + 1][2];
-          auto ldw = [&](int s) {
-#pragma unroll
-            for (int v = 0; v < 2; ++v) w[s & kAhead][v] = __ldg(Tw + 2 * s * N2 + v);
-          };
-#pragma unroll
-          for (int s = 0; s < kAhead; ++s) ldw(s);
-          waitD();
-          const int R0 = (M == 2 ? (row >> 6) * 512 : 0) + wh * 256 + nl;  // q1 = 8 wh, u
-          constexpr int RB = M == 2 ? 32 : 64;
-          const uint32_t base = sdat + t * 32768 + R0 * RB + (nmi & 1) * 8 +
-                                (((nmi >> 1) ^ (M == 2 ? (R0 >> 2) & 1 : (R0 >> 1) & 3)) << 4);
-          steps(R_, ld_seq, sum2, [&](int s, uint64_t x, uint64_t y) {
-            if (s + kAhead < 8) ldw(s + kAhead);
-            sts8(base + s * 16 * RB, mul_lazy(x, w[s & kAhead][0], R_));
-            sts8(base + (128 + s * 16) * RB, mul_lazy(y, w[s & kAhead][1], R_));
-          });
-        } else {
-          const int qm = row & (NM - 1), q1l = M == 2 ? (row >> 2) & 15 : row >> M;
-          // digit nl = 8 wh + j: every layout xors bits of nl below the first that depends on wh
-          uint32_t base;
-          int ch;  // swizzled chunk before the xor with bits of nl
-          if (M == 4) {
-            base = t * 32768 + (q1l * 16 + 8 * wh) * 128 + (qm & 1) * 8;
-            ch = qm >> 1;
-          } else if (M == 5) {
-            base = t * 32768 + (qm >> 4) * 16384 + (q1l * 16 + 8 * wh) * 128 + (qm & 1) * 8;
-            ch = (qm & 15) >> 1;
-          } else if (M == 3) {
-            base = t * 32768 + ((q1l >> 3) * 256 + (q1l & 7) * 16 + 8 * wh) * 64 + (qm & 1) * 8;
-            ch = qm >> 1;
-          } else {
-            base = t * 32768 + ((row >> 6) * 512 + (q1l >> 3) * 256 + (q1l & 7) * 16 + 8 * wh) * 32 + (qm & 1) * 8;
-            ch = qm >> 1;
-          }
-          base += sdat;
-          constexpr int RB = M >= 4 ? 128 : (M == 3 ? 64 : 32);
-          constexpr int UV = M == 4 ? 16384 : (M == 5 ? 64 * 128 : 128 * RB);
-          const ulonglong2* Tw = T2 + 8 * wh * NM + qm;
-          waitD();
-          steps(R_, ld_seq, sum2, [&](int j, uint64_t x, uint64_t y) {
-            const ulonglong2 w = __ldg(Tw + j * NM);
-            const int sw = M >= 4 ? j : (M == 3 ? (j >> 1) & 3 : (j >> 2) & 1);
-            const uint32_t a = base + j * RB + ((ch ^ sw) << 4);
-            sts8(a, mul_lazy(x, w, R_));
-            sts8(a + UV, mul_lazy(y, w, R_));
-          });
-        }
+        ep.first(t, T1, T2, waitD, none);
         doneE_smem();
       }
-      // ---- middle pass ----
 #pragma unroll 1
-      for (int t = d; t < TILES; t += 2) {  // N = 4096 forward: t = half h; N = 8192 forward: t = 2 h + s
-        const int q1l = row >> 4, nl = row & 15;
-        if (!INV) {
-          const int o0 = M == 5 ? 16 * (t & 1) + 8 * wh : (M == 4 ? 8 * wh : 0);  // first digit qm
-          const ulonglong2* Tw = T2 + o0 * 16 + nl;
-          if (M == 5)
-            waitD_both();  // both products of the half have read what the results replace
-          else
-            waitD();
-          steps(R_, ld_uv, sum2, [&](int s, uint64_t x, uint64_t y) {
-            const int oj = M == 2 ? s & 3 : s;
-            const ulonglong2 w = __ldg(Tw + oj * 16);
-            const int qm = o0 + oj, pn = nl >> 3;
-            int r3;
-            uint32_t a;
-            if (M == 5) {
-              r3 = q1l * 32 + qm;
-              a = (pn * 2 + (r3 >> 7)) * 32768 + (t >> 1) * 16384 + (r3 & 127) * 128;
-            } else if (M == 4) {
-              r3 = q1l * 16 + qm;
-              a = pn * 32768 + t * 16384 + r3 * 128;
-            } else if (M == 3) {
-              r3 = (wh * 8 + q1l) * 8 + qm;
-              a = t * 32768 + pn * 16384 + r3 * 128;
-            } else {
-              r3 = wh * 64 + ((s >> 2) * 8 + q1l) * 4 + qm;
-              a = t * 32768 + pn * 16384 + r3 * 128;
-            }
-            sts16(sdat + a + (((nl & 7) ^ (r3 & 7)) << 4), mul_lazy(x, w, R_), mul_lazy(y, w, R_));
-          });
-        } else if (M != 5) {
-          // M == 2: row tiles 2 wh (q1 = q1l) and 2 wh + 1 (q1 = 8 + q1l) of residue wh, 4 outputs each
-          const int q1 = M == 4 ? 8 * t + q1l : (M == 3 ? wh * 8 + q1l : q1l);
-          const int o0 = M == 4 ? 8 * wh : 0;  // first digit nm
-          const ulonglong2* Tw = T1 + 2 * (q1 * N2 + 16 * o0 + nl);
-          auto tw_off = [&](int s) { return M == 2 ? 2 * ((s >> 2) * 8 * N2 + 16 * (s & 3)) : 32 * s; };
-          ulonglong2 w[kAhead + 1][2];
-          auto ldw = [&](int s) {
-#pragma unroll
-            for (int v = 0; v < 2; ++v) w[s & kAhead][v] = __ldg(Tw + tw_off(s) + v);
-          };
-#pragma unroll
-          for (int s = 0; s < kAhead; ++s) ldw(s);
-          waitD();
-          const int n2 = 16 * o0 + nl;
-          const uint32_t a = sdat + t * 32768 +
-                             (M == 4 ? n2 * 128 : (M == 3 ? wh * 16384 + n2 * 128 : (wh * 64 + n2) * 128)) +
-                             ((q1l ^ (nl & 7)) << 4);
-          steps(R_, ld_uv, sum2, [&](int s, uint64_t x, uint64_t y) {
-            if (s + kAhead < 8) ldw(s + kAhead);
-            sts16(a + (M == 2 ? (s & 3) * 2048 + (s >> 2) * 16384 : s * 2048), mul_lazy(x, w[s & kAhead][0], R_),
-                  mul_lazy(y, w[s & kAhead][1], R_));
-          });
-        } else {  // N = 8192: rows of u (lanes 0 .. 63) or of v; 16 outputs each
-          const int uv = row >> 6, q1 = 4 * t + ((row >> 4) & 3), o0 = 16 * wh;
-          const ulonglong2* Tw = T1 + 2 * (q1 * N2 + 16 * o0 + nl) + uv;
-          ulonglong2 w[kAhead + 1][2];
-          auto ldw = [&](int s) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) w[s & kAhead][i] = __ldg(Tw + 32 * (2 * s + i));
-          };
-#pragma unroll
-          for (int s = 0; s < kAhead; ++s) ldw(s);
-          waitD_both();
-          const uint32_t a = sdat + (t >> 1) * 65536 + (16 * o0 + nl) * 128 + (((q1 & 7) ^ (nl & 7)) << 4) + uv * 8;
-          steps(R_, ld_seq, sum2, [&](int s, uint64_t x, uint64_t y) {
-            if (s + kAhead < 8) ldw(s + kAhead);
-            sts8(a + 2 * s * 2048, mul_lazy(x, w[s & kAhead][0], R_));
-            sts8(a + (2 * s + 1) * 2048, mul_lazy(y, w[s & kAhead][1], R_));
-          });
-        }
+      for (int t = d; t < TILES; t += 2) {  // N = 8192: both products of a half have read what the results replace
+        if (M == 5)
+          ep.middle(t, T1, T2, waitD_both, none);
+        else
+          ep.middle(t, T1, T2, waitD, none);
         doneE_smem();
       }
-      // ---- last pass: canonical results to global memory ----
 #pragma unroll 1
       for (int t = d; t < TILES; t += 2) {
         const bool last = t + 2 >= TILES;
@@ -775,55 +835,13 @@ __global__ void __launch_bounds__(kThreads, 1)
           waitD_both();  // for the loads below
         else
           waitD();
-        if (INV && last && u + 1 < u1 && (A.isrc.mode == 0 || A.isrc.mode == 2)) {
+        if (INV && last && u + 1 < u1) {
           // every product that reads this group's tiles is done: the next operand can come in
-          load_inv(u + 1);
+          load_unit(u + 1);
         }
-        if (INV) {
-          const int g = M >= 4 ? 0 : (M == 3 ? t : 2 * t + (row >> 6));
-          const int n2 = M >= 4 ? 128 * t + row : (M == 3 ? row : row & 63);
-          const bool live = g < count;
-          ulonglong2* x = A.data + (live ? item_at(r, first + g).off : 0) + 8 * wh * N2 + n2;
-          steps(R_, ld_seq, sum2, [&](int s, uint64_t a, uint64_t b) {
-            if (s == 6) doneE();  // the columns of the last step have arrived
-            if (live) x[s * N2] = make_ulonglong2(red2p(a, R_.p), red2p(b, R_.p));
-          });
-        } else {
-          // A row's results are contiguous: four neighbouring lanes take four elements of a row
-          // (64 bytes a store), so that a store instruction touches 8 lines and not 32.
-          const int rw = (warp & 3) * 32;  // rows of this warp; M == 2: all of one residue
-          const int g = M >= 4 ? 0 : (M == 3 ? t : 2 * t + (rw >> 6));
-          const int r0 = M >= 4 ? 128 * t + rw : (M == 3 ? rw : rw & 63);
-          const bool live = g < count;
-          ulonglong2* x = A.data + (live ? item_at(r, first + g).off : 0) + (r0 + (lane >> 2)) * 16 + 8 * wh + (lane & 3);
-          uint64_t z0 = 0, z1 = 0;
-          // step: 16-lane half s >> 2, group of 4 elements (s >> 1) & 1, component s & 1
-          steps(R_, [&](int s, uint32_t(&c)[16]) {
-            tmem_ld_quad(c, tl + ((uint32_t)((s >> 2) * 16) << 16) + 128 * wh + 32 * (s & 3));
-          }, [](const uint32_t* c, uint64_t& x, uint64_t& y, const Red& R_) {
-            x = col_sum(c[0], c[1], c[4], c[5], c[8], c[9], c[12], c[13], R_);
-            y = col_sum(c[2], c[3], c[6], c[7], c[10], c[11], c[14], c[15], R_);
-          }, [&](int s, uint64_t a, uint64_t b) {
-            if (s == 6) doneE();  // the columns of the last step have arrived
-            a = red2p(a, R_.p);
-            b = red2p(b, R_.p);
-            if (s & 1) {
-              ulonglong2* y = x + (s >> 2) * 256 + 4 * ((s >> 1) & 1);
-              if (live) {
-                y[0] = make_ulonglong2(z0, a);
-                y[128] = make_ulonglong2(z1, b);
-              }
-            } else {
-              z0 = a;
-              z1 = b;
-            }
-          });
-        }
+        ep.last(t, [&](int g) { return g < count ? A.data + item_at(r, first + g).off : nullptr; }, doneE);
       }
-      if (INV && u + 1 < u1) {
-        if (A.isrc.mode == 1 || A.isrc.mode == 3) load_inv(u + 1);
-        load_done();
-      }
+      if (INV && u + 1 < u1) load_done();
     }
   }
   fence_before_sync();
@@ -887,12 +905,11 @@ int launch_m(const TArgs& A, unsigned max_units, cudaStream_t st) {
   if (!INV)
     if (int rc = forward_map<M>(A, &fmap)) return rc;
   static std::atomic<unsigned long long> done{0};
-  constexpr int smem = Cfg<M>::SMEM;
-  if (int rc = ensure_smem(k_tdgt<M, INV>, smem, done)) return rc;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (sms < 1) sms = 1;
+  constexpr int smem = Cfg<M>::SMEM;
+  if (int rc = ensure_smem(k_tdgt<M, INV>, smem, done)) return rc;
   const unsigned grid = max_units < (unsigned)sms ? max_units : (unsigned)sms;
   k_tdgt<M, INV><<<grid, kThreads, smem, st>>>(A, fmap);
   return check_launch("dgt (tensor cores)");
@@ -933,7 +950,11 @@ int launch_tdgt(const Engine& e, ulonglong2* data, const ulonglong2* fsrc, const
   A.poly_stride = poly_stride;
   A.b2 = inverse && A.S == 0 ? isrc.untwist : 0;
   A.err = e.d_err;
-  const long long G = M >= 4 ? 1 : (M == 3 ? 2 : 4);
+  const long long G = M >= 4 ? 1 : (M == 3 ? 2 : 4);  // residues per unit
+  if (inverse && isrc.mode != 0 && isrc.mode != 2) {
+    set_error("dgt (tensor cores): products are formed before the transform");
+    return CP_ERR_INVALID_;
+  }
   if (rid_list && A.S > 0) {
     set_error("dgt (tensor cores): a work list needs a whole-CTA size");
     return CP_ERR_INVALID_;

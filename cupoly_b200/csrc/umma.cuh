@@ -30,15 +30,15 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
-constexpr uint32_t kWaitPolls = 1u << 20;         // each poll suspends for at most about 2 us
+constexpr uint32_t kWaitPolls = 1u << 20;         // each poll suspends for the hardware's own time limit
 constexpr uint64_t kWaitNs = 2000000000ull;       // and no wait lasts longer than 2 s
 
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(2000u)
+      : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
 }
@@ -48,7 +48,7 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatil
   uint64_t t0 = 0;
   for (uint32_t i = 0; i < kWaitPolls; ++i) {
     if (mbar_try(bar, parity)) return;
-    if ((i & 255u) == 255u) {
+    if ((i & 15u) == 15u) {
       uint64_t t;
       asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
       if (t0 == 0) t0 = t;
