@@ -15,6 +15,10 @@ __device__ __forceinline__ uint64_t pack64(uint32_t lo, uint32_t hi) {
   return r;
 }
 
+__device__ __forceinline__ double u32_to_double(uint32_t x) {  // exact, FP64 pipe only
+  return __hiloint2double(0x43300000, (int)x) - 4503599627370496.0;
+}
+
 // Per-prime constants of the epilogues.  The powers of two sit in registers: as immediates
 // the compiler turns the multiply-adds into separate shifts and adds.
 struct Red {

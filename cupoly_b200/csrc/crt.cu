@@ -10,9 +10,10 @@
 // Coefficient layout: unsigned integers of `nlimbs` 64-bit limbs, least
 // significant first, coefficient-major: uint64_t[npolys][nphi][nlimbs].
 //  * CRT: residue r of coefficient x = sum_l x_l (2^(64 l) mod q_r), a lazy
-//    192-bit dot product with one final reduction.
+//    192-bit dot product with one final reduction, or a byte matrix product.
 //  * ICRT: the mixed-radix digits d_i of X (exact, word-size), then
-//    X = d_0 + q_0 (d_1 + q_1 (d_2 + ...)) by multi-limb Horner; X in [0, Q).
+//    X = d_0 + q_0 (d_1 + q_1 (d_2 + ...)) by multi-limb Horner; X in [0, Q); or
+//    the CRT sum as a byte matrix product, from the overflow count.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -23,19 +24,21 @@
 #include "../../include/cupoly_b200.h"
 #include "launch.cuh"
 #include "product_sums.cuh"
+#include "umma.cuh"
 
 namespace cpoly {
 
 namespace {
 
+constexpr int kCrtTensor = 32;    // most limbs of cp_crt on the tensor cores (256 bytes: column sums below 2^24)
+constexpr int kIcrtTensor = 16;   // most primes of cp_icrt on the tensor cores (256 columns of tensor memory)
 constexpr int kMaxIcrt = 24;  // largest base recombined by cp_icrt (|Q|, |B| <= 24)
 
 // i / d for i < 2^16, 2 <= d <= 64, with m = ceil(2^32 / d).
 __device__ __forceinline__ int div_small(int i, uint32_t m) { return (int)__umulhi((uint32_t)i, m); }
 
-__device__ __forceinline__ void cp_async8(uint64_t* shared, const uint64_t* global) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(shared)), "l"(global)
-               : "memory");
+__device__ __forceinline__ void cp_async8(uint32_t shared, const uint64_t* global) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(shared), "l"(global) : "memory");
 }
 
 // R residues from rid on of one Gaussian element whose limbs are at s0 and s1.
@@ -77,10 +80,11 @@ __global__ void __launch_bounds__(128) k_crt(ulonglong2* __restrict__ out, const
   const int T = blockDim.x, j0 = blockIdx.x * T, nt = N - j0 < T ? N - j0 : T, row = nlimbs | 1;
   const uint64_t* c0 = coefs + ((size_t)blockIdx.y * 2 * N + j0) * nlimbs;
   const uint64_t* c1 = c0 + (size_t)N * nlimbs;
+  const uint32_t base = umma::smem_u32(s_limbs);
   for (int i = threadIdx.x; i < nt * nlimbs; i += T) {
     const int e = nlimbs == 1 ? i : div_small(i, inv_nlimbs), at = e * row + (i - e * nlimbs);
-    cp_async8(s_limbs + at, c0 + i);  // all of them in flight together
-    cp_async8(s_limbs + T * row + at, c1 + i);
+    cp_async8(base + 8 * at, c0 + i);  // all of them in flight together
+    cp_async8(base + 8 * (T * row + at), c1 + i);
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
@@ -186,6 +190,289 @@ IcrtFn icrt_kernel(int ns, std::integer_sequence<int, I...>) {
   return table[ns - 1];
 }
 
+// ---- on the tensor cores ----
+//
+// Both directions are constant linear maps of bytes (see tdgt.cu): a coefficient's limbs are its
+// row of the operand as they are, residue r has 8 columns, and byte b of limb l contributes the
+// bytes of 2^(64 l + 8 b) mod q_r.  Back, with y_i = x_i (Q/q_i)^-1 mod q_i,
+//   X = sum_i y_i (Q/q_i) - v Q,  v = floor(sum_i y_i / q_i),
+// whose limb has 8 columns, modulo 2^(64 NS); v, counted in FP64 and rounded down, is one more
+// byte (times 2^(64 NS) - Q), and at most one subtraction of Q is left.  Per output 8 column sums
+// and one fold (a carry) are left of NS products and a reduction on the integer multiply pipe.
+// A CTA of 128 threads takes 128 Gaussian elements: coefficients j and j + N are rows of two
+// tiles.  crt / icrt of 128 polynomials (us; CUDA cores below), nphi 8192, 5
+// residues (13 us of traffic each): 23 / 29 (36 / 31); 32 polynomials, nphi 16384, 12 residues (16
+// us): 29 / 40 (69 / 115).  What is left is the latency of a tile's steps, four CTAs a SM.
+struct IoTensor {
+  const uint8_t* mat;
+  int cols, tiles_per_poly, ntiles;
+  uint32_t inv_nlimbs;
+  int* err;
+};
+
+__global__ void __launch_bounds__(128, 4)
+    k_crt_tensor(ulonglong2* __restrict__ out, const uint64_t* __restrict__ coefs, int nlimbs, int N, int nres,
+                 int rid_off, const ModConst* __restrict__ mc, IoTensor io) {
+  using namespace umma;
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  __shared__ uint64_t s_bar[2];
+  __shared__ uint32_t s_slot;
+  __shared__ int s_fail;
+  const int tid = threadIdx.x;
+  const ConvShape sh{nlimbs, nres};
+  const int grp = sh.group(), ngrp = sh.groups(), cols = sh.cols();
+  const int KB = (8 * nlimbs + 31) / 32 * 32, CH = KB / 16;
+  const uint32_t sA = smem_u32(smem_raw), sB = sA + 2 * 128 * KB;
+  const uint32_t bD = smem_u32(s_bar), bB = bD + 8;
+  if (tid == 0) {
+    mbar_init(bD, 1);
+    mbar_init(bB, 1);
+    mbar_init_fence();
+    s_fail = 0;
+    mbar_expect_tx(bB, CH * cols * 16);
+    for (int ch = 0; ch < CH; ++ch)
+      bulk_load(sB + ch * cols * 16, io.mat + ((size_t)ch * io.cols + 8 * rid_off) * 16, cols * 16, bB);
+  }
+  if (tid < 32) tmem_alloc(smem_u32(&s_slot), 128);
+  auto word = [&](int comp, int row, int l) { return sA + comp * 128 * KB + (l >> 1) * 2048 + row * 16 + (l & 1) * 8; };
+  for (int l = nlimbs; l < KB / 8; ++l)
+    for (int comp = 0; comp < 2; ++comp)
+      asm volatile("st.shared.b64 [%0], %1;" ::"r"(word(comp, tid, l)), "l"(0ull) : "memory");
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = s_slot, tl = tmem + ((uint32_t)(tid & 96) << 16);
+  const uint32_t idesc = idesc_u8(128, 8 * grp);
+  const uint64_t dA = smem_desc(sA, 2048, 128, kSwzNone), dB = smem_desc(sB, cols * 16, 128, kSwzNone);
+  uint32_t k8 = 256;
+  asm volatile("" : "+r"(k8));
+  uint32_t pd = 0;
+  auto load = [&](int tile) {
+    const int poly = tile / io.tiles_per_poly, j0 = (tile % io.tiles_per_poly) * 128;
+    const uint64_t* c0 = coefs + ((size_t)poly * 2 * N + j0) * nlimbs;
+    const uint64_t* c1 = c0 + (size_t)N * nlimbs;
+    for (int i = tid; i < 128 * nlimbs; i += 128) {
+      const int e = nlimbs == 1 ? i : div_small(i, io.inv_nlimbs), l = i - e * nlimbs;
+      cp_async8(word(0, e, l), c0 + i);
+      cp_async8(word(1, e, l), c1 + i);
+    }
+  };
+  if ((int)blockIdx.x < io.ntiles) load(blockIdx.x);
+  bool first = true;
+  for (int tile = blockIdx.x; tile < io.ntiles; tile += gridDim.x) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    fence_async_smem();
+    fence_before_sync();
+    __syncthreads();  // every row is written, and the last tile's products are read
+    auto issue = [&](int g) {
+      if (tid == 0) {
+        fence_after_sync();
+        for (int comp = 0; comp < 2; ++comp)
+          for (int ks = 0; ks < KB / 32; ++ks)
+            mma_u8(tmem + 64 * comp, dA + (comp * 128 * KB + ks * 4096) / 16, dB + (ks * 2 * cols + g * grp * 8), idesc,
+                   ks > 0);
+        mma_commit(bD);
+      }
+    };
+    if (first) mbar_wait(bB, 0, &s_fail);
+    first = false;
+    issue(0);
+    const int poly = tile / io.tiles_per_poly, j = (tile % io.tiles_per_poly) * 128 + tid;
+    ulonglong2* o = out + (size_t)poly * nres * N + j;
+    for (int g = 0; g < ngrp; ++g) {
+      const int t0 = g * grp, t1 = t0 + grp < nres ? t0 + grp : nres;
+      mbar_wait(bD, pd & 1, &s_fail);
+      ++pd;
+      fence_after_sync();
+      // the operand has been read: the next tile's limbs are on their way during the sums
+      if (g == ngrp - 1 && tile + (int)gridDim.x < io.ntiles) load(tile + gridDim.x);
+      uint32_t c0[16], c1[16];
+      auto ld = [&](int t, uint32_t(&c)[16]) { tmem_ld8x2(c, tl + 8 * (t - t0), tl + 64 + 8 * (t - t0)); };
+      auto one = [&](int t, const uint32_t(&c)[16]) {
+        const uint64_t p = mc[rid_off + t].p;
+        const Red R{p, (uint32_t)((1ull << 63) - p), k8, k8 << 8};
+        o[(size_t)t * N] = make_ulonglong2(red2p(col_sum(c, R), p), red2p(col_sum(c + 8, R), p));
+      };
+      ld(t0, c0);
+#pragma unroll 1
+      for (int t = t0; t < t1; t += 2) {  // the next residue's columns are on their way while one is summed
+        tmem_ld_wait(c0);
+        if (t + 1 < t1) ld(t + 1, c1);
+        one(t, c0);
+        if (t + 1 < t1) {
+          tmem_ld_wait(c1);
+          if (t + 2 < t1) ld(t + 2, c0);
+          one(t + 1, c1);
+        }
+      }
+      if (g + 1 < ngrp) {
+        fence_before_sync();
+        __syncthreads();  // the group's products are read
+        issue(g + 1);
+      }
+    }
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (tid < 32) tmem_dealloc(tmem, 128);
+  if (tid == 0 && s_fail) atomicExch(io.err, 2);
+}
+
+// Shapes and constants of cp_icrt's matrix: K bytes (NS residues and the count), columns (limbs,
+// a multiple of 16), then the words (Q/q_i)^-1 mod q_i, their Shoup quotients, 1/q_i as FP64 and
+// the limbs of Q.
+__host__ __device__ constexpr int icrt_kbytes(int ns) { return (8 * ns + 1 + 31) / 32 * 32; }
+__host__ __device__ constexpr int icrt_cols(int ns) { return (8 * ns + 15) / 16 * 16; }
+constexpr size_t icrt_bytes(int ns) { return (size_t)icrt_kbytes(ns) * icrt_cols(ns) + 4 * 8 * (size_t)ns; }
+
+template <int NS>
+__global__ void __launch_bounds__(128, NS <= 8 ? 4 : 2)
+    k_icrt_tensor(uint64_t* __restrict__ coefs, int nlimbs, const ulonglong2* __restrict__ in, int N, int src_off,
+                  const ModConst* __restrict__ mc, IoTensor io) {
+  using namespace umma;
+  constexpr int KB = icrt_kbytes(NS), CH = KB / 16, COLS = icrt_cols(NS), HALF = NS <= 8 ? 64 : 128;
+  constexpr int ROW = NS | 1;  // words between the staged coefficients, in the operand's own place
+  static_assert(ROW * 8 <= KB, "staging");
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  __shared__ uint64_t s_bar[2];
+  __shared__ uint32_t s_slot;
+  __shared__ int s_fail;
+  const int tid = threadIdx.x;
+  const uint32_t sA = smem_u32(smem_raw), sB = sA + 2 * 128 * KB;
+  const uint32_t bD = smem_u32(s_bar), bB = bD + 8;
+  if (tid == 0) {
+    mbar_init(bD, 1);
+    mbar_init(bB, 1);
+    mbar_init_fence();
+    s_fail = 0;
+    mbar_expect_tx(bB, KB * COLS);
+    bulk_load(sB, io.mat, KB * COLS, bB);
+  }
+  if (tid < 32) tmem_alloc(smem_u32(&s_slot), 2 * HALF);
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = s_slot, tl = tmem + ((uint32_t)(tid & 96) << 16);
+  const uint32_t idesc = idesc_u8(128, COLS);
+  const uint64_t dA = smem_desc(sA, 2048, 128, kSwzNone), dB = smem_desc(sB, COLS * 16, 128, kSwzNone);
+  const uint64_t* inv = reinterpret_cast<const uint64_t*>(io.mat + KB * COLS);
+  const uint64_t *inv_s = inv + NS, *recip = inv + 2 * NS, *Q = inv + 3 * NS;
+  uint32_t k8 = 256;
+  asm volatile("" : "+r"(k8));
+  const uint32_t k16 = k8 << 8;
+  ulonglong2 x[NS];
+  auto load = [&](int tile) {
+    const ulonglong2* p = in + (size_t)(tile / io.tiles_per_poly) * NS * N + (tile % io.tiles_per_poly) * 128 + tid;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) x[i] = p[(size_t)i * N];
+  };
+  if ((int)blockIdx.x < io.ntiles) load(blockIdx.x);
+  uint32_t pd = 0;
+  for (int tile = blockIdx.x; tile < io.ntiles; tile += gridDim.x) {
+#pragma unroll
+    for (int comp = 0; comp < 2; ++comp) {
+      uint64_t y[NS + 1];
+      double f = -0x1p-40;  // FP64 errors are below 2^-45: v is never too large, and one too small at most
+#pragma unroll
+      for (int i = 0; i < NS; ++i) {
+        y[i] = shoup_mul(comp ? x[i].y : x[i].x, __ldg(inv + i), __ldg(inv_s + i), mc[src_off + i].p);
+        const double c = __longlong_as_double(__ldg(recip + i));
+        f = __fma_rn(u32_to_double((uint32_t)y[i]), c, f);
+        f = __fma_rn(u32_to_double((uint32_t)(y[i] >> 32)), c * 4294967296.0, f);
+      }
+      y[NS] = f > 0.0 ? (uint64_t)(uint32_t)__double2int_rd(f) : 0;
+      const uint32_t row = sA + comp * 128 * KB + tid * 16;
+#pragma unroll
+      for (int ch = 0; ch < CH; ++ch) {
+        const uint64_t lo = 2 * ch <= NS ? y[2 * ch <= NS ? 2 * ch : 0] : 0;
+        const uint64_t hi = 2 * ch + 1 <= NS ? y[2 * ch + 1 <= NS ? 2 * ch + 1 : 0] : 0;
+        asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(row + ch * 2048), "l"(lo), "l"(hi) : "memory");
+      }
+    }
+    fence_async_smem();
+    fence_before_sync();
+    __syncthreads();  // every row is written, and the last tile's products are read
+    if (pd == 0) mbar_wait(bB, 0, &s_fail);
+    if (tid == 0) {
+      fence_after_sync();
+#pragma unroll
+      for (int comp = 0; comp < 2; ++comp)
+#pragma unroll
+        for (int ks = 0; ks < KB / 32; ++ks)
+          mma_u8(tmem + HALF * comp, dA + (comp * 128 * KB + ks * 4096) / 16, dB + ks * 2 * COLS, idesc, ks > 0);
+      mma_commit(bD);
+    }
+    const int poly = tile / io.tiles_per_poly, j0 = (tile % io.tiles_per_poly) * 128;
+    if (tile + (int)gridDim.x < io.ntiles) load(tile + gridDim.x);  // on their way during the products
+    mbar_wait(bD, pd & 1, &s_fail);
+    ++pd;
+    fence_after_sync();
+#pragma unroll 1
+    for (int comp = 0; comp < 2; ++comp) {
+      uint64_t X[NS], D[NS];
+      uint32_t carry = 0;
+      uint32_t c[2][16];
+      tmem_ld16(c[0], tl + HALF * comp);
+#pragma unroll
+      for (int l = 0; l < NS; ++l) {  // two limbs a load; the columns past the last limb are zero
+        const uint32_t* s = c[(l >> 1) & 1] + 8 * (l & 1);
+        if ((l & 1) == 0) {
+          tmem_ld_wait(c[(l >> 1) & 1]);
+          if (l + 2 < NS) tmem_ld16(c[((l >> 1) + 1) & 1], tl + HALF * comp + 8 * (l + 2));
+        }
+        // as col_sum: a 17-bit carry fits on top of a word of two columns
+        const uint32_t a0 = s[1] * k8 + s[0] + carry, a1 = s[3] * k8 + s[2];
+        const uint32_t a2 = s[5] * k8 + s[4], a3 = s[7] * k8 + s[6];
+        const uint64_t t = mad_wide(a1, k16, pack64(a0, a2));
+        const uint64_t h = mad_wide(a3, k16, (uint64_t)(t >> 32));
+        X[l] = pack64((uint32_t)t, (uint32_t)h);
+        carry = (uint32_t)(h >> 32);
+      }
+      uint64_t borrow = 0;
+#pragma unroll
+      for (int l = 0; l < NS; ++l) {
+        const uint64_t q = __ldg(Q + l), d = X[l] - q;
+        D[l] = d - borrow;
+        borrow = (X[l] < q) | (d < borrow);
+      }
+      const uint32_t at = sA + comp * 128 * KB + tid * ROW * 8;
+#pragma unroll
+      for (int l = 0; l < NS; ++l)
+        asm volatile("st.shared.b64 [%0], %1;" ::"r"(at + 8 * l), "l"(borrow ? X[l] : D[l]) : "memory");
+    }
+    fence_before_sync();
+    __syncthreads();
+    for (int comp = 0; comp < 2; ++comp) {
+      uint64_t* o = coefs + ((size_t)poly * 2 * N + (size_t)comp * N + j0) * nlimbs;
+      const uint64_t* sx = reinterpret_cast<const uint64_t*>(smem_raw + comp * 128 * KB);
+      for (int i = tid; i < 128 * nlimbs; i += 128) {
+        const int e = nlimbs == 1 ? i : div_small(i, io.inv_nlimbs), l = i - e * nlimbs;
+        o[i] = l < NS ? sx[e * ROW + l] : 0;
+      }
+    }
+    __syncthreads();  // the staged coefficients are read
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (tid < 32) tmem_dealloc(tmem, 2 * HALF);
+  if (tid == 0 && s_fail) atomicExch(io.err, 2);
+}
+
+using IcrtTensorFn = void (*)(uint64_t*, int, const ulonglong2*, int, int, const ModConst*, IoTensor);
+template <int... I>
+IcrtTensorFn icrt_tensor_kernel(int ns, std::integer_sequence<int, I...>) {
+  static constexpr IcrtTensorFn table[] = {k_icrt_tensor<I + 1>...};
+  return table[ns - 1];
+}
+
+int io_ctas(int smem_bytes, int most_per_sm) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int fit = 220 * 1024 / (smem_bytes + 1024);
+  return (sms > 0 ? sms : 1) * std::max(1, std::min(fit, most_per_sm));
+}
+
 __global__ void __launch_bounds__(256) k_icrt_t(uint64_t* __restrict__ coefs, int nlimbs,
                                                 const ulonglong2* __restrict__ in, int N) {
   const int jj = blockIdx.x * blockDim.x + threadIdx.x;
@@ -216,6 +503,86 @@ const uint64_t* base_primes(const Engine& e, int base, uint64_t* tmp) {
 
 }  // namespace
 
+// The matrices and constants of k_crt_tensor and k_icrt_tensor.
+int build_io_tables(Engine& e) {
+  const int R = e.k + e.kl;
+  std::vector<uint8_t> io;
+  e.io_cols = 0;
+  if (!e.ckks_prec) {  // column sums fold by 2^63 = c
+    e.io_cols = 8 * (R + 24);  // a base's columns are read up to a multiple of its groups
+    io.assign((size_t)kCrtTensor / 2 * e.io_cols * 16, 0);
+    for (int r = 0; r < R; ++r) {
+      uint64_t f = 1;  // 2^(8 kb) mod p
+      for (int kb = 0; kb < 8 * kCrtTensor; ++kb) {
+        uint8_t* at = io.data() + ((size_t)(kb >> 4) * e.io_cols + 8 * r) * 16 + (kb & 15);
+        for (int j = 0; j < 8; ++j) at[16 * j] = (uint8_t)(f >> (8 * j));
+        f = h_mul(f, 256, e.mconst[r]);
+      }
+    }
+  }
+  for (int v = 0; v < 2; ++v) {
+    const int ns = v ? e.kl : e.k;
+    if (ns > kIcrtTensor) continue;
+    const uint64_t* p = e.primes.data() + (v ? e.k : 0);
+    const ModConst* m = e.mconst.data() + (v ? e.k : 0);
+    const int kb_n = icrt_kbytes(ns), cols = icrt_cols(ns);
+    e.io_icrt[v] = io.size();
+    io.resize(io.size() + ((icrt_bytes(ns) + 127) & ~(size_t)127), 0);
+    uint8_t* mat = io.data() + e.io_icrt[v];
+    uint64_t* words = reinterpret_cast<uint64_t*>(mat + (size_t)kb_n * cols);
+    auto product = [&](int skip) {  // of the base's primes, in ns limbs
+      std::vector<uint64_t> x(ns, 0);
+      x[0] = 1;
+      for (int i = 0; i < ns; ++i) {
+        if (i == skip) continue;
+        uint64_t carry = 0;
+        for (int l = 0; l < ns; ++l) {
+          const unsigned __int128 w = (unsigned __int128)x[l] * p[i] + carry;
+          x[l] = (uint64_t)w;
+          carry = (uint64_t)(w >> 64);
+        }
+      }
+      return x;
+    };
+    auto put = [&](int kb, const std::vector<uint64_t>& x, int shift) {  // bytes of x 2^(8 shift) mod 2^(64 ns)
+      for (int c = shift; c < 8 * ns; ++c)
+        mat[(size_t)(kb >> 4) * cols * 16 + (size_t)c * 16 + (kb & 15)] = (uint8_t)(x[(c - shift) >> 3] >> (8 * ((c - shift) & 7)));
+    };
+    const std::vector<uint64_t> Q = product(-1);
+    std::vector<uint64_t> neg(ns);  // 2^(64 ns) - Q
+    uint64_t carry = 1;
+    for (int l = 0; l < ns; ++l) {
+      neg[l] = ~Q[l] + carry;
+      carry = carry && neg[l] == 0;
+    }
+    put(8 * ns, neg, 0);
+    for (int i = 0; i < ns; ++i) {
+      const std::vector<uint64_t> x = product(i);
+      for (int b = 0; b < 8; ++b) put(8 * i + b, x, b);
+      uint64_t f = 1;
+      for (int l = 0; l < ns; ++l)
+        if (l != i) f = h_mul(f, p[l] % p[i], m[i]);
+      const uint64_t w = h_invmod(f, p[i]);
+      const double rec = 1.0 / (double)p[i];
+      words[i] = w;
+      words[ns + i] = h_shoup(w, m[i]);
+      std::memcpy(words + 2 * ns + i, &rec, 8);
+      words[3 * ns + i] = Q[i];
+    }
+  }
+  if (io.empty()) return 0;
+  cudaError_t err = cudaMalloc(&e.d_io, io.size());
+  if (err != cudaSuccess) {
+    set_error(std::string("cudaMalloc failed for engine tables: ") + cudaGetErrorString(err));
+    return 4;
+  }
+  if ((err = cudaMemcpy(e.d_io, io.data(), io.size(), cudaMemcpyHostToDevice)) != cudaSuccess) {
+    set_error(std::string("table upload failed: ") + cudaGetErrorString(err));
+    return 2;
+  }
+  return 0;
+}
+
 }  // namespace cpoly
 
 using namespace cpoly;
@@ -240,6 +607,22 @@ int cp_crt(const cp_engine* h, void* out, const uint64_t* coefs, int nlimbs, int
   const int nres = e.n_residues(base);
   if (npolys == 0) return CP_OK;
   CRT_REQUIRE((long long)npolys * nres <= 65535, "cp_crt: npolys x residues exceeds 65535");
+  if (e.d_io && e.io_cols && nlimbs <= kCrtTensor && e.N >= 128) {
+    const int kb = (8 * nlimbs + 31) / 32 * 32;
+    const long long tiles = (long long)npolys * (e.N / 128);
+    const int smem = std::max(2 * 128 * kb + kb * ConvShape{nlimbs, nres}.cols(), 46 * 1024);
+    // Below some 16 K tile x limb x residue steps the CUDA cores are faster (us, 5 limbs and residues:
+    // 512 tiles 6.8 there and 7.7 here, 4096 tiles 36 and 23; 12: 128 tiles 7.9 and 7.2, 512 tiles 20 and 11).
+    if (smem <= 200 * 1024 && tiles * nlimbs * nres >= 16384) {
+      static std::atomic<unsigned long long> done{0};
+      if (int rc = ensure_smem(k_crt_tensor, 200 * 1024, done)) return rc;
+      const IoTensor io{e.d_io, e.io_cols, e.N / 128, (int)tiles, inv_small(nlimbs), e.d_err};
+      k_crt_tensor<<<(unsigned)std::min<long long>(tiles, io_ctas(smem, 4)), 128, smem,
+                     reinterpret_cast<cudaStream_t>(stream)>>>(reinterpret_cast<ulonglong2*>(out), coefs, nlimbs, e.N,
+                                                               nres, e.rid_offset(base), e.d_mc, io);
+      return check_launch("cp_crt");
+    }
+  }
   // elements per block: the limbs take at most 48 KB
   const int T = nlimbs <= 23 ? 128 : (nlimbs <= 47 ? 64 : 32);
   const unsigned bx = (unsigned)((e.N + T - 1) / T), groups = (unsigned)((nres + 3) / 4);
@@ -269,6 +652,22 @@ int cp_icrt(const cp_engine* h, uint64_t* coefs, int nlimbs, const void* in, int
     return check_launch("cp_icrt");
   }
   CRT_REQUIRE(ns <= kMaxIcrt, "cp_icrt: base larger than 24 primes");
+  if (e.d_io && ns <= kIcrtTensor && e.N >= 128) {
+    const long long tiles = (long long)npolys * (e.N / 128);
+    // The CUDA cores' chain grows with the square of the base (us: 12 residues 128 tiles 15 there and 6.0
+    // here, 2048 tiles 115 and 40; 5 residues 512 tiles 6.0 and 7.2, 4096 tiles 32 and 29).
+    if (ns >= 8 || tiles * ns * ns >= 32768) {
+      const int per = ns <= 8 ? 4 : 2;
+      const int smem = std::max(2 * 128 * icrt_kbytes(ns) + icrt_kbytes(ns) * icrt_cols(ns), per == 4 ? 46 * 1024 : 80 * 1024);
+      IcrtTensorFn fn = icrt_tensor_kernel(ns, std::make_integer_sequence<int, kIcrtTensor>());
+      static std::atomic<unsigned long long> done[kIcrtTensor + 1];
+      if (int rc = ensure_smem(fn, smem, done[ns])) return rc;
+      const IoTensor io{e.d_io + e.io_icrt[base == CP_QBASE ? 0 : 1], 0, e.N / 128, (int)tiles, inv_small(nlimbs), e.d_err};
+      fn<<<(unsigned)std::min<long long>(tiles, io_ctas(smem, per)), 128, smem, st>>>(coefs, nlimbs, src, e.N,
+                                                                                      e.rid_offset(base), e.d_mc, io);
+      return check_launch("cp_icrt");
+    }
+  }
   const uint64_t* inv = e.d_hps + (base == CP_QBASE ? e.ho.qb_inv : e.ho.bq_inv);
   const uint64_t* inv_s = e.d_hps + (base == CP_QBASE ? e.ho.qb_inv_s : e.ho.bq_inv_s);
   icrt_kernel(ns, std::make_integer_sequence<int, kMaxIcrt>())<<<dim3((e.N + 63) / 64, npolys), 128, 0, st>>>(

@@ -191,6 +191,11 @@ struct Engine {
   // byte matrices of the base conversions of prescaled residues (hps.cu): Q -> B, t/Q scaling, B -> Q
   uint8_t* d_cmat = nullptr;
   size_t cmat_off[3] = {0, 0, 0};
+  // coefficient I/O on the tensor cores (crt.cu): byte matrix of cp_crt (residue columns; 63-bit
+  // primes), then per base (Q, B) of at most kIcrtTensor primes the matrix and constants of cp_icrt
+  uint8_t* d_io = nullptr;
+  int io_cols = 0;
+  size_t io_icrt[2] = {0, 0};
   int* d_err = nullptr;            // device-side error flag (sampler rejection exhaustion)
   int hps_force_exact = 0;         // 1: every base conversion and scaling takes its exact path (tests)
 
@@ -215,6 +220,7 @@ const char* last_error();
 
 // table construction (tables.cu)
 int build_tables(Engine& e);
+int build_io_tables(Engine& e);      // crt.cu
 int build_tensor_tables(Engine& e);  // tdgt_tables.cu; after the plans are placed
 void free_tables(Engine& e);
 

@@ -133,11 +133,6 @@ struct Fast {
   const uint64_t* invd;           // per source: 1/s_i as IEEE-754 double bits
 };
 
-// FP64 overflow count: sum_i y_i / s_i = v + X/S.  Returns whether v (and,
-// with `half`, the side of 1/2 of X/S) is certain.
-__device__ __forceinline__ double u32_to_double(uint32_t x) {  // exact, FP64 pipe only
-  return __hiloint2double(0x43300000, (int)x) - 4503599627370496.0;
-}
 
 // cuPoly's lift: X in [0, S) is read as X - S when X / S >= 1 - FPERROR (see
 // lift_threshold_digits in tables.cu); this is the fraction side of that test.
@@ -152,6 +147,8 @@ constexpr double kLiftFrac = 1.0 - 1e-9;
 // whose values are small signed integers (fractions within 2^-40 of 0 or 1), therefore takes
 // the fast path.
 
+// FP64 overflow count: sum_i y_i / s_i = v + X/S.  Returns whether v (and,
+// with `half`, the side of 1/2 of X/S) is certain.
 template <int NS>
 __device__ __forceinline__ bool fast_v(const uint64_t (&y)[NS], const uint64_t* __restrict__ invd, bool half, int& v,
                                        bool& above, bool lift = false, bool* neg = nullptr) {

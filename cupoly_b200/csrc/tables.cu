@@ -686,6 +686,10 @@ int build_tables(Engine& e) {
       return 2;
     }
   }
+  if (const int rc = build_io_tables(e)) {
+    free_tables(e);
+    return rc;
+  }
   if (const int rc = build_tensor_tables(e)) {
     free_tables(e);
     return rc;
@@ -702,6 +706,8 @@ void free_tables(Engine& e) {
   e.d_ttab = nullptr;
   if (e.d_cmat) cudaFree(e.d_cmat);
   e.d_cmat = nullptr;
+  if (e.d_io) cudaFree(e.d_io);
+  e.d_io = nullptr;
   e.d_err = nullptr;
   e.d_tab = nullptr;
   e.d_mc = nullptr;
