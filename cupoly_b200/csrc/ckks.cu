@@ -11,12 +11,15 @@
 //  * xi / rho: x_i B^-1 mod q_i and x_i B mod q_i (xi_ckks_rns_rid,
 //    rho_ckks_rns_rid).
 // Q_l = q_0 ... q_l; Q is the first 63-bit prime followed by primes of the
-// precision bucket in descending order, so x_l < q_l < q_i for i < l.  Every
-// multiply is by a constant (Shoup product with a precomputed quotient), so
-// nothing here depends on the prime's form.  The definitions above are
-// integer-exact; the results are the same whatever the reduction order.
+// precision bucket in descending order, so x_l < q_l < q_i for i < l.  Single
+// multiplies are by constants (Shoup products with precomputed quotients), the
+// sums are reduced once (const_dot).  The definitions above are integer-exact;
+// the results are the same whatever the reduction order.
 #include "../../include/cupoly_b200.h"
+#include <utility>
+
 #include "launch.cuh"
+#include "product_sums.cuh"
 
 namespace cpoly {
 
@@ -30,48 +33,75 @@ struct CkArgs {
   int N, k, kl, level;
 };
 
-// B residues of the coefficient-domain Q residues 0..level (rows of N elements).
-// Polynomial blockIdx.y at strides out_stride / in_stride (elements).
-__global__ void __launch_bounds__(128) k_ckks_raise(ulonglong2* __restrict__ outB, const ulonglong2* __restrict__ inQ,
-                                                    CkArgs a, int o_inv, int o_inv_s, int o_m, int o_m_s,
-                                                    long long out_stride, long long in_stride) {
+// sum_i y[i] c[i stride] mod m.p for residues y[i] of different primes of one base and c[] < m.p:
+// one sum of products, one reduction.  An engine has a single 63-bit prime (q_0) and at most 24
+// others per base, all below 2^56: the primes of a base sum to less than 2^64, so the sum of products
+// stays below m.p 2^64, what the Montgomery step wants.
+template <int NS>
+__device__ __forceinline__ uint64_t const_dot(const uint64_t (&y)[NS], const uint64_t* __restrict__ c, int stride,
+                                              const ModConst& m) {
+  ProductSum<true> sum;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) sum.mac(y[i], __ldg(c + i * stride));
+  if (m.pm) {
+    const uint32_t c0 = (uint32_t)((1ull << 63) - m.p);
+    return canon(sum.fold(c0), c0, m.p);
+  }
+  uint64_t lo, hi;
+  sum.words(lo, hi);
+  return gen_red(hi, lo, m);
+}
+
+// The base conversions keep a coefficient's source residues in registers: their number is a
+// template argument (indexed by a loop over the level they lay in local memory).  They are bound by
+// the integer multiply pipe: raising of 16 polynomials at nphi 16384, 7 residues to 9, 37 us
+// before, 21 us so with the copy below.
+
+// B residues of the coefficient-domain Q residues 0..NS-1 (rows of N elements), and the Q rows of
+// the result, a copy of `dgt` (k rows).  Polynomial blockIdx.y at strides out_stride / in_stride
+// (elements) of the QB result and of both inputs.  The copy is memory traffic under the
+// conversion's arithmetic; as a 2-D copy of its own it took 18 us of the above call.
+template <int NS>
+__global__ void __launch_bounds__(128) k_ckks_raise(ulonglong2* __restrict__ out, const ulonglong2* __restrict__ inQ,
+                                                    const ulonglong2* __restrict__ dgt, CkArgs a, int o_inv,
+                                                    int o_inv_s, int o_m, long long out_stride, long long in_stride) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= a.N) return;
-  outB += blockIdx.y * out_stride;
-  inQ += blockIdx.y * in_stride;
-  const int l = a.level;
-  uint64_t tr[kMaxCk], ti[kMaxCk];
-  for (int i = 0; i <= l; ++i) {
+  out += blockIdx.y * out_stride + j;
+  inQ += blockIdx.y * in_stride + j;
+  dgt += blockIdx.y * in_stride + j;
+  constexpr int l = NS - 1;
+  uint64_t tr[NS], ti[NS];
+#pragma unroll
+  for (int i = 0; i < NS; ++i) {
     const uint64_t q = a.mc[i].p;
-    const ulonglong2 x = inQ[(size_t)i * a.N + j];
+    const ulonglong2 x = inQ[(size_t)i * a.N];
     const uint64_t c = __ldg(a.H + o_inv + l * a.k + i), cs = __ldg(a.H + o_inv_s + l * a.k + i);
     tr[i] = shoup_mul(x.x, c, cs, q);
     ti[i] = shoup_mul(x.y, c, cs, q);
   }
+  for (int i = 0; i < a.k; ++i) out[(size_t)i * a.N] = dgt[(size_t)i * a.N];
+  out += (size_t)a.k * a.N;
   for (int jb = 0; jb < a.kl; ++jb) {
-    const uint64_t b = a.mc[a.k + jb].p;
-    uint64_t ar = 0, ai = 0;
-    for (int i = 0; i <= l; ++i) {
-      const size_t w = ((size_t)l * a.k + i) * a.kl + jb;
-      const uint64_t c = __ldg(a.H + o_m + w), cs = __ldg(a.H + o_m_s + w);
-      ar = add_mod(ar, shoup_mul(tr[i], c, cs, b), b);  // tr[i] < q_i < 2^64: any input
-      ai = add_mod(ai, shoup_mul(ti[i], c, cs, b), b);
-    }
-    outB[(size_t)jb * a.N + j] = make_ulonglong2(ar, ai);
+    const ModConst m = a.mc[a.k + jb];
+    const uint64_t* c = a.H + o_m + l * a.k * a.kl + jb;
+    out[(size_t)jb * a.N] = make_ulonglong2(const_dot(tr, c, a.kl, m), const_dot(ti, c, a.kl, m));
   }
 }
 
 // Q residues 0..level of the coefficient-domain QB polynomial; higher Q rows untouched.
 // Polynomial blockIdx.y at strides out_stride / in_stride (elements).
+template <int NS>
 __global__ void __launch_bounds__(128) k_ckks_reduce(ulonglong2* __restrict__ outQ, const ulonglong2* __restrict__ inQB,
-                                                     CkArgs a, int o_bi, int o_bi_s, int o_bq, int o_bq_s, int o_ib,
-                                                     int o_ib_s, long long out_stride, long long in_stride) {
+                                                     CkArgs a, int o_bi, int o_bi_s, int o_bq, int o_ib, int o_ib_s,
+                                                     long long out_stride, long long in_stride) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= a.N) return;
   outQ += blockIdx.y * out_stride;
   inQB += blockIdx.y * in_stride;
-  uint64_t sr[kMaxCk], si[kMaxCk];
-  for (int jb = 0; jb < a.kl; ++jb) {
+  uint64_t sr[NS], si[NS];
+#pragma unroll
+  for (int jb = 0; jb < NS; ++jb) {
     const uint64_t b = a.mc[a.k + jb].p;
     const ulonglong2 y = inQB[(size_t)(a.k + jb) * a.N + j];
     const uint64_t c = __ldg(a.H + o_bi + jb), cs = __ldg(a.H + o_bi_s + jb);
@@ -79,17 +109,27 @@ __global__ void __launch_bounds__(128) k_ckks_reduce(ulonglong2* __restrict__ ou
     si[jb] = shoup_mul(y.y, c, cs, b);
   }
   for (int i = 0; i <= a.level; ++i) {
-    const uint64_t q = a.mc[i].p;
-    uint64_t vr = 0, vi = 0;
-    for (int jb = 0; jb < a.kl; ++jb) {
-      const uint64_t c = __ldg(a.H + o_bq + jb * a.k + i), cs = __ldg(a.H + o_bq_s + jb * a.k + i);
-      vr = add_mod(vr, shoup_mul(sr[jb], c, cs, q), q);
-      vi = add_mod(vi, shoup_mul(si[jb], c, cs, q), q);
-    }
+    const ModConst m = a.mc[i];
+    const uint64_t q = m.p;
+    const uint64_t vr = const_dot(sr, a.H + o_bq + i, a.k, m);
+    const uint64_t vi = const_dot(si, a.H + o_bq + i, a.k, m);
     const ulonglong2 x = inQB[(size_t)i * a.N + j];
     const uint64_t c = __ldg(a.H + o_ib + i), cs = __ldg(a.H + o_ib_s + i);
     outQ[(size_t)i * a.N + j] = make_ulonglong2(shoup_mul(x.x + q - vr, c, cs, q), shoup_mul(x.y + q - vi, c, cs, q));
   }
+}
+
+using RaiseFn = void (*)(ulonglong2*, const ulonglong2*, const ulonglong2*, CkArgs, int, int, int, long long, long long);
+using ReduceFn = void (*)(ulonglong2*, const ulonglong2*, CkArgs, int, int, int, int, int, long long, long long);
+template <int... I>
+RaiseFn raise_kernel(int ns, std::integer_sequence<int, I...>) {
+  static constexpr RaiseFn table[] = {k_ckks_raise<I + 1>...};
+  return table[ns - 1];
+}
+template <int... I>
+ReduceFn reduce_kernel(int ns, std::integer_sequence<int, I...>) {
+  static constexpr ReduceFn table[] = {k_ckks_reduce<I + 1>...};
+  return table[ns - 1];
 }
 
 // x_i <- (x_i - x_l) q_l^-1 mod q_i for i < level; polynomial blockIdx.y.
@@ -160,12 +200,11 @@ static int ckks_raise(const cp_engine* h, void* out_qb, const void* in_q, int le
   ulonglong2* out = reinterpret_cast<ulonglong2*>(out_qb);
   ulonglong2* w = reinterpret_cast<ulonglong2*>(ws);
   const long long qsz = (long long)e.k * e.N, qbsz = (long long)(e.k + e.kl) * e.N;
-  cudaError_t err = cudaMemcpy2DAsync(out, qbsz * 16, in_q, qsz * 16, qsz * 16, npolys, cudaMemcpyDeviceToDevice, st);
-  if (err != cudaSuccess) return cuda_fail(name, err);
   if (int rc = launch_dgt_part(e, w, in_q, 0, level + 1, npolys, qsz, true, st)) return rc;  // Q_l, coefficients
   const auto& o = e.ho;
-  k_ckks_raise<<<dim3((e.N + 127) / 128, npolys), 128, 0, st>>>(out + qsz, w, args(e, level), o.ck_qlqi_inv,
-                                                                 o.ck_qlqi_inv_s, o.ck_qlqi_b, o.ck_qlqi_b_s, qbsz, qsz);
+  raise_kernel(level + 1, std::make_integer_sequence<int, kMaxCk>())<<<dim3((e.N + 127) / 128, npolys), 128, 0, st>>>(
+      out, w, reinterpret_cast<const ulonglong2*>(in_q), args(e, level), o.ck_qlqi_inv, o.ck_qlqi_inv_s, o.ck_qlqi_b,
+      qbsz, qsz);
   if (int rc = check_launch(name)) return rc;
   return launch_dgt_part(e, out + qsz, nullptr, e.k, e.kl, npolys, qbsz, false, st);
 }
@@ -187,9 +226,8 @@ static int ckks_reduce(const cp_engine* h, void* out_q, const void* in_qb, int l
   if (int rc = launch_dgt_part(e, w + qsz, in + qsz, e.k, e.kl, npolys, qbsz, true, st)) return rc;
   const auto& o = e.ho;
   ulonglong2* out = reinterpret_cast<ulonglong2*>(out_q);
-  k_ckks_reduce<<<dim3((e.N + 127) / 128, npolys), 128, 0, st>>>(out, w, args(e, level), o.ck_bbj_inv, o.ck_bbj_inv_s,
-                                                                  o.ck_bbj_q, o.ck_bbj_q_s, o.ck_binv_q, o.ck_binv_q_s,
-                                                                  qsz, qbsz);
+  reduce_kernel(e.kl, std::make_integer_sequence<int, kMaxCk>())<<<dim3((e.N + 127) / 128, npolys), 128, 0, st>>>(
+      out, w, args(e, level), o.ck_bbj_inv, o.ck_bbj_inv_s, o.ck_bbj_q, o.ck_binv_q, o.ck_binv_q_s, qsz, qbsz);
   if (int rc = check_launch(name)) return rc;
   return launch_dgt_part(e, out, nullptr, 0, level + 1, npolys, qsz, false, st);
 }

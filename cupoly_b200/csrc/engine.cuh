@@ -180,9 +180,9 @@ struct Engine {
     // CKKS (only when ckks_prec != 0); every constant with its Shoup companion
     int ck_inv_ql, ck_inv_ql_s;    // q_l^-1 mod q_i, [l][i]
     int ck_qlqi_inv, ck_qlqi_inv_s;  // (Q_l / q_i)^-1 mod q_i, [l][i]; Q_l = q_0 ... q_l
-    int ck_qlqi_b, ck_qlqi_b_s;    // (Q_l / q_i) mod b_j, [l][i][j]
+    int ck_qlqi_b;                 // (Q_l / q_i) mod b_j, [l][i][j]
     int ck_bbj_inv, ck_bbj_inv_s;  // (B / b_j)^-1 mod b_j, [j]
-    int ck_bbj_q, ck_bbj_q_s;      // (B / b_j) mod q_i, [j][i]
+    int ck_bbj_q;                  // (B / b_j) mod q_i, [j][i]
     int ck_binv_q, ck_binv_q_s;    // B^-1 mod q_i, [i]
     int ck_b_q, ck_b_q_s;          // B mod q_i, [i]
   } ho{};

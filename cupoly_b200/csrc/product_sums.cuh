@@ -22,6 +22,16 @@ struct ProductSum {
         : "l"(a), "l"(b));
   }
 
+  // the sum when it is below 2^128
+  __device__ __forceinline__ void words(uint64_t& lo, uint64_t& hi) const {
+    uint32_t r1, r2, r3;
+    asm("add.cc.u32 %0, %3, %6;\n\taddc.cc.u32 %1, %4, %7;\n\taddc.u32 %2, %5, %8;"
+        : "=&r"(r1), "=&r"(r2), "=&r"(r3)
+        : "r"(e1), "r"(e2), "r"(e3), "r"(o0), "r"(o1), "r"(o2));
+    lo = pack64(e0, r1);
+    hi = pack64(r2, r3);
+  }
+
   // the sum mod p, any representative below 2^64: folds by 2^64 = 2 c, the last one's carry again
   __device__ __forceinline__ uint64_t fold(uint32_t c) const {
     const uint32_t C = 2 * c;

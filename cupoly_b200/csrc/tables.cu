@@ -579,7 +579,7 @@ int build_tables(Engine& e) {
   }
   if (e.ckks_prec) {
     const int k = e.k, kl = e.kl;
-    std::vector<uint64_t> a, as, b, bs, c, cs, d, ds, f, fs, g, gs, h, hs;
+    std::vector<uint64_t> a, as, b, bs, c, d, ds, f, g, gs, h, hs;
     for (int l = 0; l < k; ++l)
       for (int i = 0; i < k; ++i) {
         const uint64_t qi = Q[i];
@@ -593,7 +593,7 @@ int build_tables(Engine& e) {
           uint64_t mb = 1 % B[j];  // Q_l / q_i mod b_j
           for (int u = 0; u <= l; ++u)
             if (u != i) mb = h_mulmod(mb, Q[u] % B[j], B[j]);
-          push_pair(i <= l ? mb : 0, B[j], c, cs);
+          c.push_back(i <= l ? mb : 0);
         }
       }
     for (int j = 0; j < kl; ++j) {
@@ -605,7 +605,7 @@ int build_tables(Engine& e) {
         uint64_t mq = 1 % Q[i];
         for (int u = 0; u < kl; ++u)
           if (u != j) mq = h_mulmod(mq, B[u] % Q[i], Q[i]);
-        push_pair(mq, Q[i], f, fs);
+        f.push_back(mq);
       }
     }
     for (int i = 0; i < k; ++i) {
@@ -618,11 +618,9 @@ int build_tables(Engine& e) {
     e.ho.ck_qlqi_inv = append(b);
     e.ho.ck_qlqi_inv_s = append(bs);
     e.ho.ck_qlqi_b = append(c);
-    e.ho.ck_qlqi_b_s = append(cs);
     e.ho.ck_bbj_inv = append(d);
     e.ho.ck_bbj_inv_s = append(ds);
     e.ho.ck_bbj_q = append(f);
-    e.ho.ck_bbj_q_s = append(fs);
     e.ho.ck_binv_q = append(g);
     e.ho.ck_binv_q_s = append(gs);
     e.ho.ck_b_q = append(h);
