@@ -418,8 +418,7 @@ int cp_polymul(const cp_engine* h, void* c, const void* a, const void* b, int ba
   ulonglong2* wa = reinterpret_cast<ulonglong2*>(workspace);
   ulonglong2* wb = wa + (size_t)npolys * e.n_residues(base) * e.N;
   cudaStream_t st = S(stream);
-  if (int rc = launch_dgt_ex(e, wa, a, nullptr, base, npolys, 0, false, st)) return rc;
-  if (int rc = launch_dgt_ex(e, wb, b, nullptr, base, npolys, 0, false, st)) return rc;
+  if (int rc = launch_dgt_pair(e, wa, a, b, base, npolys, st)) return rc;
   InvSrc is{};
   is.p[0] = wa;
   is.npairs = 1;

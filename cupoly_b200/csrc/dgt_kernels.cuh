@@ -179,6 +179,10 @@ __device__ __forceinline__ ulonglong2* fwd_dst(const DgtArgs& A, ulonglong2* dat
   if (!A.scatter[0]) return data + poly * poly_stride;
   return poly == 0 ? A.scatter[0] : poly == 1 ? A.scatter[1] : A.scatter[2];
 }
+// The second source's distance (DgtArgs::src_polys).
+__device__ __forceinline__ long long src_shift(const DgtArgs& A, int poly) {
+  return A.src_polys && poly >= A.src_polys ? A.src_shift : 0;
+}
 
 // One middle/late forward pass (I >= 1), full radix 2^LOGR, data in smem.
 template <int LOGNC, int LOGR, int I>
@@ -427,8 +431,10 @@ __global__ void __launch_bounds__((1 << LOGNC) >> LOGR, (dgt_min_blocks<LOGNC, L
            ((size_t)(ub & ((1u << S) - 1)) << LOGNC);
   };
   for (unsigned ub = blockIdx.x; ub < nunits; ub += gridDim.x) {
-  if (dgt_prefetches<LOGNC, LOGR, CL>() && tid == 0 && ub + gridDim.x < nunits)
-    prefetch_l2(in_base + unit_off(ub + gridDim.x), NC * 16u);
+  if (dgt_prefetches<LOGNC, LOGR, CL>() && tid == 0 && ub + gridDim.x < nunits) {
+    const unsigned un = ub + gridDim.x;
+    prefetch_l2(in_base + unit_off(un) + src_shift(A, (int)(un >> S) / nres), NC * 16u);
+  }
   const int pr = (int)(ub >> S);
   const int r = pr % nres;
   const int rid = A.rid_list ? A.rid_list[pr] : rid_off + r;
@@ -437,7 +443,7 @@ __global__ void __launch_bounds__((1 << LOGNC) >> LOGR, (dgt_min_blocks<LOGNC, L
   const size_t off = unit_off(ub);
   const int poly = pr / nres;
   ulonglong2* x = fwd_dst(A, data, poly, poly_stride) + (off - (size_t)poly * poly_stride);
-  const ulonglong2* xs = src_base ? src_base + off : x;  // in place: the output's own place
+  const ulonglong2* xs = src_base ? src_base + off + src_shift(A, poly) : x;  // in place: the output's own place
   for (int j = tid; j < R; j += T) srad[j] = tab[A.L.off_rad + j];
   stage_twiddles<LOGNC, LOGR>(stw, tab, A.L.off_fwd);
   __syncthreads();
@@ -680,7 +686,7 @@ __global__ void __launch_bounds__(256)
   const uint64_t p = A.mc[rid].p;
   const ulonglong2* tab = A.tab + (size_t)rid * A.stride;
   ulonglong2* x = (INV ? data + poly * poly_stride : fwd_dst(A, data, poly, poly_stride)) + ((size_t)r << (logNc + S));
-  const ulonglong2* xs = src_base ? src_base + poly * poly_stride + ((size_t)r << (logNc + S)) : x;
+  const ulonglong2* xs = src_base ? src_base + poly * poly_stride + src_shift(A, poly) + ((size_t)r << (logNc + S)) : x;
   constexpr int K = 1 << S;
   uint64_t xr[K], xi[K];
   const int R = 1 << logR;

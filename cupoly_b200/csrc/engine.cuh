@@ -66,6 +66,10 @@ struct DgtArgs {
   const ModConst* mc;      // per engine residue
   const int* rid_list;     // work list: residue i of the data uses engine prime rid_list[i] (nullptr: base order)
   ulonglong2* scatter[3];  // forward output of polynomials 0..2 (scatter[0] nullptr: at `data`)
+  // Out of place, polynomials from src_polys on are read src_shift elements further: a second
+  // source array (0: there is none).
+  int src_polys;
+  long long src_shift;
 };
 
 // Tensor-core DGT tables (tdgt.cu): byte offsets inside one residue's block.  The matrices are

@@ -289,7 +289,7 @@ class Engine:
         return torch.empty(((n + 15) // 16, 2), dtype=torch.int64, device="cuda")
 
     def polymul(self, c, a, b, base, workspace, npolys=None, stream=None):
-        """c = a b mod (x^nphi + 1) per residue, coefficient domain in and out (fused: 3 launches)."""
+        """c = a b mod (x^nphi + 1) per residue, coefficient domain in and out (fused; see cp_polymul)."""
         n = c.shape[0] if npolys is None else npolys
         ws = self._ws(workspace, _lib.lib().cp_polymul_workspace_bytes(self._h, base, n))
         call("cp_polymul", self._h, *self._bufs(base, n, c=c, a=a, b=b), base, n, ws, _stream(stream))

@@ -162,9 +162,10 @@ int cp_mul_list(const cp_engine* e, void* c, const void* a, const void* b, const
 /* ---- fused negacyclic polymul, coefficient domain in and out (no counterpart in cuPoly,
  *      whose poly_mul composes upload DGTs, mul_dgt and a download IDGT,
  *      src/arithmetic/polynomial.cu:892-914 with :105-188): c = a b mod (x^nphi + 1, q_r)
- *      per residue, as forward DGT of a and b out of place into the workspace, then an
- *      inverse DGT that forms the Gaussian products while loading (3 launches).  c may
- *      alias a or b.  cp_polymul: npolys polynomials over `base`, workspace of
+ *      per residue, as forward DGTs of a and b out of place into the workspace (one
+ *      launch for small cp_polymul calls), then an inverse DGT that forms the Gaussian
+ *      products while loading, or a product kernel and an inverse DGT on the tensor
+ *      cores.  c may alias a or b.  cp_polymul: npolys polynomials over `base`, workspace of
  *      cp_polymul_workspace_bytes bytes.  cp_polymul_list: work-list form (see
  *      cp_dgt_list), wa and wb each nlist x N x 16 bytes. ---- */
 size_t cp_polymul_workspace_bytes(const cp_engine* e, int base, int npolys);
