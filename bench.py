@@ -517,9 +517,10 @@ def run_ours(args, D: Dist):
         D.barrier()
     ms = D.max(ev0.elapsed_time(ev1))
     value = D.world * P * args.steps / (ms / 1e3)
-    # inverse DGT (gather) + Q->B + forward DGT(B) + 2 inverse DGTs with the tensor
-    # product fused in + complex scaling + B->Q + forward DGT(Q) (nphi <= 16384: one kernel per DGT)
-    launches_per_step = 8
+    # inverse DGT (gather) + Q->B + forward DGT(B) + 2 inverse DGTs of the tensor product + complex
+    # scaling + B->Q + forward DGT(Q) (nphi <= 16384: one kernel per DGT); the products are two
+    # kernels of their own on the tensor cores, part of the inverses on the CUDA cores
+    launches_per_step = 10 if e.get_tensor() else 8
 
     # ---- e2e: host-resident batches through the public API (StreamedBFV: copy-in,
     # chain and copy-out of consecutive batches overlap on three streams); every
@@ -617,8 +618,9 @@ def run_ours(args, D: Dist):
     dgt_ms = ev0.elapsed_time(ev1) / reps
     dgt_bytes = 2 * 16 * e.N * 4 * P * K_B  # read + write every Gaussian element once
     achieved = dgt_bytes / (dgt_ms / 1e3) / 1e9
-    # integer roofline of the same launch: algorithmic Shoup multiplies and modular
-    # adds at the measured peak rates of those primitives on this GPU
+    # integer roofline of the same launch on the CUDA cores: algorithmic Shoup multiplies and modular
+    # adds at the measured peak rates of those primitives on this GPU (the tensor cores do the
+    # butterflies, so their launch can be faster than this model)
     from cupoly_b200.engine import dgt_op_counts, int_peaks
     peaks_int = int_peaks()
     ops = dgt_op_counts(e.N)
@@ -662,7 +664,7 @@ def run_ours(args, D: Dist):
     torch.cuda.synchronize()
     polymul_plain_value = NPp / (ev0.elapsed_time(ev1) / 1e3)
 
-    # ---- batched: coefficient domain in and out, fused cp_polymul (3 launches per batch), two consecutive
+    # ---- batched: coefficient domain in and out, fused cp_polymul (4 launches per batch), two consecutive
     # batches in flight on two streams (batch.PipelinedPolymul), each with its own output
     from cupoly_b200.batch import PipelinedPolymul
     ppm = PipelinedPolymul(e1, QBase, NPm, lanes=2)
@@ -725,9 +727,10 @@ def run_ours(args, D: Dist):
     mixed_ms = mixed_forms[best]
     mixed = {"config": "1024 products, nphi uniform in {2048, 4096, 8192, 16384}, k uniform in 1..8 (seeded), "
                        "2 batches in flight; fastest of three forms: %s" % best,
-             "form": {"sequence": "one CUDA graph, per size group a fused cp_polymul_list (3 launches)",
+             "form": {"sequence": "one CUDA graph, per size group a fused cp_polymul_list (3 launches; 4 on the tensor cores)",
                       "branches": "the same graph with one parallel branch per size group",
                       "tiles": "one persistent launch (cp_polymul_tiles) over a work list of tiles"}[best],
+             # transform launches; on the tensor cores the products are one more per size group
              "launches_per_batch": mixed_launches[best],
              "polymul_per_s": round(1024 / (mixed_ms / 1e3), 1), "ms_per_batch": round(mixed_ms, 3),
              "ms_per_batch_by_form": {k_: round(v_, 4) for k_, v_ in mixed_forms.items()},
@@ -879,7 +882,7 @@ def run_ours(args, D: Dist):
             "plain_cxx": percall_cxx,
             "batched_over_plain": round(value / D.world / plain_value, 2),
             "polymul": ({"value": round(polymul_value, 1), "unit": "polymul/s",
-                         "config": "nphi=4096, k=2, batch 1024 (fused: 2 forward DGTs, inverse with products on load), 2 batches in flight",
+                         "config": "nphi=4096, k=2, batch 1024 (fused: 2 forward DGTs, products, inverse), 2 batches in flight",
                          "algorithmic_GB_per_s": round(polymul_value * 24 * 4096 * 2 / 1e9, 1),
                          "frac_hbm": round(polymul_value * 24 * 4096 * 2 / 1e9 / hbm_peak, 4),
                          "plain_value": round(polymul_plain_value, 1),
@@ -897,10 +900,10 @@ def run_ours(args, D: Dist):
                          # dram__bytes_read.sum + dram__bytes_write.sum of this launch (same
                          # kernel, 3072 residues of N = 4096) from one ncu capture; writes read low
                          # because dirty lines are still in L2 when the kernel ends
-                         "traffic": 346929920 if (e.N == 4096 and 4 * P * K_B == 3072) else None,
+                         "traffic": 350900000 if (e.N == 4096 and 4 * P * K_B == 3072 and e.get_tensor()) else None,
                          "traffic_source": "ncu capture",
-                         "kernel": "k_dgt_fwd (forward DGT, %d residues of N=%d per launch, timed alone)" %
-                                   (4 * P * K_B, e.N),
+                         "kernel": "%s (forward DGT, %d residues of N=%d per launch, timed alone)" %
+                                   ("k_tdgt" if e.get_tensor() else "k_dgt_fwd", 4 * P * K_B, e.N),
                          "peak_source": "MEASURED_PEAKS.json hbm_gbs (burst)" if peaks else "fallback",
                          "int": int_roof},
             "cupoly_gpu": cupoly_gpu,

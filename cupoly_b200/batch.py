@@ -191,6 +191,8 @@ class MixedPolymul:
         self.graph.replay()
 
     def launches_per_run(self) -> int:
+        """Transform launches of one run, with the products in the inverse; a group large enough for the
+        tensor cores takes one more, its products."""
         return 1 if self.mode == "tiles" else 3 * len(self.groups)
 
     def algorithmic_bytes(self) -> int:
