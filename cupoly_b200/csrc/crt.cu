@@ -31,7 +31,7 @@ namespace cpoly {
 namespace {
 
 constexpr int kCrtTensor = 32;    // most limbs of cp_crt on the tensor cores (256 bytes: column sums below 2^24)
-constexpr int kIcrtTensor = 16;   // most primes of cp_icrt on the tensor cores (256 columns of tensor memory)
+constexpr int kIcrtFirst = 5, kIcrtTensor = 16;  // primes of cp_icrt on the tensor cores (at most 256 columns of tensor memory)
 constexpr int kMaxIcrt = 24;  // largest base recombined by cp_icrt (|Q|, |B| <= 24)
 
 // i / d for i < 2^16, 2 <= d <= 64, with m = ceil(2^32 / d).
@@ -461,8 +461,8 @@ __global__ void __launch_bounds__(128, NS <= 8 ? 4 : 2)
 using IcrtTensorFn = void (*)(uint64_t*, int, const ulonglong2*, int, int, const ModConst*, IoTensor);
 template <int... I>
 IcrtTensorFn icrt_tensor_kernel(int ns, std::integer_sequence<int, I...>) {
-  static constexpr IcrtTensorFn table[] = {k_icrt_tensor<I + 1>...};
-  return table[ns - 1];
+  static constexpr IcrtTensorFn table[] = {k_icrt_tensor<I + kIcrtFirst>...};
+  return table[ns - kIcrtFirst];
 }
 
 int io_ctas(int smem_bytes, int most_per_sm) {
@@ -522,7 +522,7 @@ int build_io_tables(Engine& e) {
   }
   for (int v = 0; v < 2; ++v) {
     const int ns = v ? e.kl : e.k;
-    if (ns > kIcrtTensor) continue;
+    if (ns < kIcrtFirst || ns > kIcrtTensor) continue;
     const uint64_t* p = e.primes.data() + (v ? e.k : 0);
     const ModConst* m = e.mconst.data() + (v ? e.k : 0);
     const int kb_n = icrt_kbytes(ns), cols = icrt_cols(ns);
@@ -652,14 +652,15 @@ int cp_icrt(const cp_engine* h, uint64_t* coefs, int nlimbs, const void* in, int
     return check_launch("cp_icrt");
   }
   CRT_REQUIRE(ns <= kMaxIcrt, "cp_icrt: base larger than 24 primes");
-  if (e.d_io && ns <= kIcrtTensor && e.N >= 128) {
+  if (e.d_io && ns >= kIcrtFirst && ns <= kIcrtTensor && e.N >= 128) {
     const long long tiles = (long long)npolys * (e.N / 128);
     // The CUDA cores' chain grows with the square of the base (us: 12 residues 128 tiles 15 there and 6.0
-    // here, 2048 tiles 115 and 40; 5 residues 512 tiles 6.0 and 7.2, 4096 tiles 32 and 29).
+    // here, 2048 tiles 115 and 40; 6 residues 1024 tiles 13 and 10.5; 5 residues 512 tiles 6.0 and 7.2,
+    // 2048 tiles 16.9 and 15.6); up to 4 residues it is short (4 residues 4096 tiles 21 and 25).
     if (ns >= 8 || tiles * ns * ns >= 32768) {
       const int per = ns <= 8 ? 4 : 2;
       const int smem = std::max(2 * 128 * icrt_kbytes(ns) + icrt_kbytes(ns) * icrt_cols(ns), per == 4 ? 46 * 1024 : 80 * 1024);
-      IcrtTensorFn fn = icrt_tensor_kernel(ns, std::make_integer_sequence<int, kIcrtTensor>());
+      IcrtTensorFn fn = icrt_tensor_kernel(ns, std::make_integer_sequence<int, kIcrtTensor - kIcrtFirst + 1>());
       static std::atomic<unsigned long long> done[kIcrtTensor + 1];
       if (int rc = ensure_smem(fn, smem, done[ns])) return rc;
       const IoTensor io{e.d_io + e.io_icrt[base == CP_QBASE ? 0 : 1], 0, e.N / 128, (int)tiles, inv_small(nlimbs), e.d_err};

@@ -196,7 +196,7 @@ struct Engine {
   uint8_t* d_cmat = nullptr;
   size_t cmat_off[3] = {0, 0, 0};
   // coefficient I/O on the tensor cores (crt.cu): byte matrix of cp_crt (residue columns; 63-bit
-  // primes), then per base (Q, B) of at most kIcrtTensor primes the matrix and constants of cp_icrt
+  // primes), then per base (Q, B) of a size that cp_icrt takes there its matrix and constants
   uint8_t* d_io = nullptr;
   int io_cols = 0;
   size_t io_icrt[2] = {0, 0};

@@ -392,6 +392,13 @@ int pw_dot_batch(const Engine& e, void* c, const void* a, const void* b, int n, 
     return CP_ERR_INVALID_;
   }
   if (npolys <= 0) return CP_OK_;
+  // (polynomial, residue) rows over y, split over z in whole polynomials when needed
+  long long gz = 1;
+  while ((long long)npolys * nres / gz > 65535 || npolys % gz) ++gz;
+  if (gz > 65535) {
+    set_error("dot_batch: batch too large");
+    return CP_ERR_INVALID_;
+  }
   // few terms against shared b: every prime of a BFV engine has 63 bits
   if (b_shared && n <= kDotHeld && e.ckks_prec == 0) {
     using Fn = void (*)(const u2*, const u2*, u2*, int, int, int, int, const ModConst*);
@@ -401,23 +408,15 @@ int pw_dot_batch(const Engine& e, void* c, const void* a, const void* b, int n, 
     // twelve blocks for each of 148 SMs (with 6 and 12 of them the above takes 25.5 us, with 20 26,
     // with 40 29: each starts with a load of b), each with a run of polynomials
     const long long rows = (long long)bx * nres;
-    long long gz = (148LL * 12 + rows - 1) / rows;
-    if (gz > npolys) gz = npolys;
-    if (gz > 65535) gz = 65535;
-    table[n - 1]<<<dim3(bx, nres, (unsigned)gz), 128, 0, st>>>(CU2(a), CU2(b), U2(c), e.N, nres, e.rid_offset(base),
+    long long runs = (148LL * 12 + rows - 1) / rows;
+    if (runs > npolys) runs = npolys;
+    table[n - 1]<<<dim3(bx, nres, (unsigned)runs), 128, 0, st>>>(CU2(a), CU2(b), U2(c), e.N, nres, e.rid_offset(base),
                                                                npolys, e.d_mc);
     return check_launch("dot_batch");
   }
   const int threads = 256;
   int bx = (e.N + threads - 1) / threads;
   if (bx > 4096) bx = 4096;
-  // (polynomial, residue) rows over y, split over z in whole polynomials when needed
-  long long gz = 1;
-  while ((long long)npolys * nres / gz > 65535 || npolys % gz) ++gz;
-  if (gz > 65535) {
-    set_error("dot_batch: batch too large");
-    return CP_ERR_INVALID_;
-  }
   const dim3 grid(bx, (unsigned)((long long)npolys / gz * nres), (unsigned)gz);
   k_dot_batch<<<grid, threads, 0, st>>>(CU2(a), CU2(b), U2(c), n, b_shared ? 1 : 0, e.N, nres, e.rid_offset(base),
                                         e.d_mc);
