@@ -370,7 +370,11 @@ int cp_engine_check(const cp_engine* h, void* stream) {
   if (flag) {
     cudaMemsetAsync(h->e.d_err, 0, sizeof(int), S(stream));
     cudaStreamSynchronize(S(stream));
-    set_error("a kernel reported an error (sampler rejection limit reached)");
+    std::string what;
+    if (flag & kErrSampler) what += ", sampler rejection limit reached";
+    if (flag & kErrWait) what += ", a wait inside a tensor-core kernel ran out: results since the last check are invalid";
+    if (flag & kErrTile) what += ", a work-list tile outside its group was skipped";
+    set_error("a kernel reported an error: " + (what.empty() ? "code " + std::to_string(flag) : what.substr(2)));
     return CP_ERR_DEVICE;
   }
   return CP_OK;

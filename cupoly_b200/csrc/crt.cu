@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(128, 4)
   fence_before_sync();
   __syncthreads();
   if (tid < 32) tmem_dealloc(tmem, 128);
-  if (tid == 0 && s_fail) atomicExch(io.err, 2);
+  if (tid == 0 && s_fail) atomicOr(io.err, kErrWait);
 }
 
 // Shapes and constants of cp_icrt's matrix: K bytes (NS residues and the count), columns (limbs,
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(128, NS <= 8 ? 4 : 2)
   fence_before_sync();
   __syncthreads();
   if (tid < 32) tmem_dealloc(tmem, 2 * HALF);
-  if (tid == 0 && s_fail) atomicExch(io.err, 2);
+  if (tid == 0 && s_fail) atomicOr(io.err, kErrWait);
 }
 
 using IcrtTensorFn = void (*)(uint64_t*, int, const ulonglong2*, int, int, const ModConst*, IoTensor);

@@ -200,7 +200,7 @@ struct Engine {
   uint8_t* d_io = nullptr;
   int io_cols = 0;
   size_t io_icrt[2] = {0, 0};
-  int* d_err = nullptr;            // device-side error flag (sampler rejection exhaustion)
+  int* d_err = nullptr;            // device-side error flag: DeviceError bits
   int hps_force_exact = 0;         // 1: every base conversion and scaling takes its exact path (tests)
 
   int n_residues(int base) const;
@@ -216,6 +216,13 @@ struct ConvShape {
   __host__ __device__ int group() const { return ((ndst + groups() - 1) / groups() + 1) & ~1; }
   __host__ __device__ int cols() const { return 8 * group() * groups(); }
   __host__ __device__ int bytes() const { return kbytes() * cols(); }
+};
+
+// What a kernel reports through the engine's error flag (cp_engine_check).
+enum DeviceError : int {
+  kErrSampler = 1,  // a sampler's rejection limit
+  kErrWait = 2,     // a wait of a tensor-core kernel ran out (umma.cuh)
+  kErrTile = 4,     // a work-list tile outside its group
 };
 
 // thread-local error reporting

@@ -768,7 +768,7 @@ __global__ void __launch_bounds__(128, 4)
   fence_before_sync();
   __syncthreads();
   if (tid < 32) tmem_dealloc(tmem, 128);
-  if (tid == 0 && s_fail) atomicExch(tc.err, 2);
+  if (tid == 0 && s_fail) atomicOr(tc.err, kErrWait);
 }
 
 struct SimpleArgs {

@@ -3,9 +3,11 @@
 // arithmetic.  cuPoly tests its device functions directly
 // (TestDGT.{mod, addmod, submod, mulmod, powmod, GIAdd, GISub, GIMul},
 // tests/unit_tests/test_bfv_mode.cu:243-438); this entry point gives the same
-// reach to the primitives behind the C ABI.
+// reach to the primitives behind the C ABI.  Beside them, the bounded wait of the
+// tensor-core kernels (umma.cuh) on a barrier that nothing reaches.
 #include "../../include/cupoly_b200.h"
 #include "launch.cuh"
+#include "umma.cuh"
 
 namespace {
 
@@ -58,7 +60,31 @@ __global__ void __launch_bounds__(256) k_modarith(int op, const uint64_t* __rest
   }
 }
 
+__global__ void __launch_bounds__(32) k_wait_test(int* err) {
+  using namespace umma;
+  __shared__ uint64_t s_bar;
+  __shared__ int s_fail;
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&s_bar), 1);
+    mbar_init_fence();
+    s_fail = 0;
+  }
+  __syncthreads();
+  mbar_wait(smem_u32(&s_bar), 0, &s_fail);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_fail) atomicOr(err, kErrWait);
+}
+
 }  // namespace
+
+extern "C" int cp_wait_test(const cp_engine* h, void* stream) {
+  if (!h) {
+    set_error("cp_wait_test: NULL engine");
+    return CP_ERR_INVALID;
+  }
+  k_wait_test<<<1, 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(h->e.d_err);
+  return check_launch("cp_wait_test");
+}
 
 extern "C" int cp_modarith_eval(int op, const uint64_t* a, const uint64_t* b, const uint64_t* c, uint64_t* out,
                                 long long n, uint64_t p, void* stream) {

@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     const bool ok = tl.lg >= 0 && tl.lg < 4 && args.g[tl.lg].rid != nullptr && tl.count >= 1 &&
                     tl.count <= (8 >> tl.lg) && tl.row0 >= 0 && tl.row0 + tl.count <= args.g[tl.lg].rows;
     if (!ok) {
-      if (threadIdx.x == 0) atomicExch(args.err, 1);
+      if (threadIdx.x == 0) atomicOr(args.err, kErrTile);
       continue;
     }
     switch (tl.lg) {

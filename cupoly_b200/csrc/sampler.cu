@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(256) k_sample(ulonglong2* __restrict__ out, co
           ok1 = true;
         }
       }
-      if (!(ok0 && ok1)) atomicExch(err, 1);
+      if (!(ok0 && ok1)) atomicOr(err, kErrSampler);
       out[(size_t)r * N + j] = make_ulonglong2(val[0], val[1]);
     }
     return;
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(256) k_sample(ulonglong2* __restrict__ out, co
   const int nphi_log = 31 - __clz(2 * N);
   const bool ok0 = small_value(kind, (uint32_t)j, sid, k0, k1, nphi_log, v0);
   const bool ok1 = small_value(kind, (uint32_t)(j + N), sid, k0, k1, nphi_log, v1);
-  if (!(ok0 && ok1)) atomicExch(err, 1);
+  if (!(ok0 && ok1)) atomicOr(err, kErrSampler);
   for (int r = 0; r < nres; ++r) {
     const uint64_t p = mc[rid_off + r].p;
     out[(size_t)r * N + j] = make_ulonglong2(lift(v0, p), lift(v1, p));
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(256) k_sample_hw(ulonglong2* __restrict__ out,
         }
       }
       if (!placed) {
-        atomicExch(err, 1);
+        atomicOr(err, kErrSampler);
         pos[i] = -1;
       }
     }

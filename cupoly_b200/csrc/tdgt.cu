@@ -847,7 +847,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   fence_before_sync();
   __syncthreads();
   if (warp == kEpiWarps) tmem_dealloc(tmem, 512);
-  if (tid == 0 && s_fail) atomicExch(A.err, 2);
+  if (tid == 0 && s_fail) atomicOr(A.err, kErrWait);
 }
 
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

@@ -139,7 +139,16 @@ int cp_engine_set_nthroot(cp_engine* e, const uint64_t* xi);
 int cp_engine_get_nthroot(const cp_engine* e, uint64_t* xi_out);
 /* bytes of scratch the composite calls below need */
 size_t cp_workspace_bytes(const cp_engine* e);
-/* read and clear the engine's device error flag (synchronises `stream`) */
+/* Read and clear the engine's device error flag (synchronises `stream`); CP_ERR_DEVICE with a
+ * message for each cause.  The calls below return before their kernels end, so what a kernel
+ * finds comes this way:
+ *   sampler (cp_sample*): a coefficient reached the rejection limit;
+ *   tile list (cp_polymul_tiles): a tile outside its group was skipped;
+ *   tensor-core kernels (from nphi 256 on, any call that transforms, converts between bases or
+ *     reads or writes integer coefficients: cp_dgt*, cp_polymul*, cp_sample* with to_dgt, cp_bfv_mul*,
+ *     cp_crt, cp_icrt and the composites): a wait for a copy or a product ran out after about
+ *     2 s on the device.  It cannot happen in a working program; if it does, the results written since the
+ *     last check are invalid. */
 int cp_engine_check(const cp_engine* e, void* stream);
 /* the engine's error flag, copied into flag_host (page-locked host memory) on `stream` behind
  * the work already queued there, without waiting: nonzero once the copy has completed means
@@ -316,6 +325,9 @@ enum cp_modop {
 };
 int cp_modarith_eval(int op, const uint64_t* a, const uint64_t* b, const uint64_t* c, uint64_t* out, long long n,
                      uint64_t p, void* stream);
+/* One warp waits, as the tensor-core kernels do, on a barrier that nothing reaches: after about 2 s it
+ * gives up and the engine's error flag is set (for tests of the error path). */
+int cp_wait_test(const cp_engine* e, void* stream);
 
 /* ---- CKKS operations (CKKS engines only), DGT domain in and out, level l in [0, k)
  *      (rescale: [1, k)); Q_l = q_0 ... q_l.  They replace fast_conv_Q_to_B /
