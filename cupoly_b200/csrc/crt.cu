@@ -314,6 +314,7 @@ __global__ void __launch_bounds__(128, 4)
   }
   fence_before_sync();
   __syncthreads();
+  settle(&s_fail);
   if (tid < 32) tmem_dealloc(tmem, 128);
   if (tid == 0 && s_fail) atomicOr(io.err, kErrWait);
 }
@@ -454,6 +455,7 @@ __global__ void __launch_bounds__(128, NS <= 8 ? 4 : 2)
   }
   fence_before_sync();
   __syncthreads();
+  settle(&s_fail);
   if (tid < 32) tmem_dealloc(tmem, 2 * HALF);
   if (tid == 0 && s_fail) atomicOr(io.err, kErrWait);
 }

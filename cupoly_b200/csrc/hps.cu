@@ -767,6 +767,7 @@ __global__ void __launch_bounds__(128, 4)
   }
   fence_before_sync();
   __syncthreads();
+  settle(&s_fail);
   if (tid < 32) tmem_dealloc(tmem, 128);
   if (tid == 0 && s_fail) atomicOr(tc.err, kErrWait);
 }

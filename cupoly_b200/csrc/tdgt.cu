@@ -846,6 +846,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   fence_before_sync();
   __syncthreads();
+  settle(&s_fail);
   if (warp == kEpiWarps) tmem_dealloc(tmem, 512);
   if (tid == 0 && s_fail) atomicOr(A.err, kErrWait);
 }

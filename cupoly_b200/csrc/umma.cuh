@@ -1,9 +1,9 @@
 // tcgen05 building blocks of the tensor-core kernels (sm_100a): 8-bit unsigned integer
 // matrix products with 32-bit accumulators in tensor memory, mbarriers, bulk copies.
 //
-// Every wait is bounded: after kWaitPolls unsuccessful polls the wait gives up, the
+// Every wait is bounded: after kWaitPolls unsuccessful polls or kWaitNs the wait gives up, the
 // block's `fail` word is set and later waits return at once, so a block always reaches its
-// end, frees its tensor memory and reports through the engine's error flag.
+// end (settle), frees its tensor memory and reports through the engine's error flag.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -31,7 +31,9 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 }
 
 constexpr uint32_t kWaitPolls = 1u << 20;         // each poll suspends for the hardware's own time limit
-constexpr uint64_t kWaitNs = 2000000000ull;       // and no wait lasts longer than 2 s
+constexpr uint64_t kWaitNs = 2000000000ull;       // and no wait lasts longer than 2 s,
+constexpr uint32_t kWaitLeast = 1u << 10;         // except for these polls: the clock runs on while the context is
+                                                  // switched out, the copies and products waited for do not
 
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -44,7 +46,7 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 }
 // Waits until the phase of the given parity has completed; see the file comment for the bound.
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatile int* fail) {
-  if (mbar_try(bar, parity)) return;
+  if (mbar_try(bar, parity) || *fail) return;
   uint64_t t0 = 0;
   for (uint32_t i = 0; i < kWaitPolls; ++i) {
     if (mbar_try(bar, parity)) return;
@@ -52,10 +54,16 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatil
       uint64_t t;
       asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
       if (t0 == 0) t0 = t;
-      if (*fail || t - t0 > kWaitNs) break;
+      if (*fail || (i > kWaitLeast && t - t0 > kWaitNs)) break;
     }
   }
   *fail = 1;
+}
+// At a block's end, after a barrier of its threads and before its memory passes on: copies and
+// products may still be in flight if a wait ran out, and get 0.1 s to land.
+__device__ __forceinline__ void settle(const volatile int* fail) {
+  if (*fail)
+    for (int i = 0; i < 100; ++i) __nanosleep(1000000);
 }
 
 // Tensor memory: `ncols` (a power of two >= 32) 32-bit columns of 128 lanes, by one whole warp.
