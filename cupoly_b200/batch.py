@@ -30,7 +30,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .engine import FORWARD, INVERSE, QBase, Engine, _ptr, _stream, from_u64, to_u64
+from .engine import FORWARD, INVERSE, QBase, Engine, _ptr, _stream, from_u64
 from ._lib import call
 
 
@@ -131,7 +131,8 @@ class MixedPolymul:
     def result(self, i: int) -> np.ndarray:
         nphi, row = self.where[i]
         k = self.specs[i][1]
-        x = to_u64(self.groups[nphi]["c"][row:row + k])
+        g = self.groups[nphi]
+        x = g["engine"].download(g["c"][row:row + k])
         return np.concatenate([x[..., 0], x[..., 1]], axis=-1)
 
     # ---- execution ----
@@ -341,7 +342,9 @@ class StreamedBFV:
     device-to-host copy of batch i - 1 at the same time over `nbuf` device buffer
     sets, so throughput is bound by the slowest of the three instead of their
     sum.  A copy-in waits only for the chain that last read its input buffers,
-    and a chain only for the copy-out that last read its output buffer.
+    and a chain only for the copy-out that last read its output buffer.  Nothing here
+    waits on the host: engine.check() after the outputs have arrived raises what a kernel
+    has reported.
     """
 
     def __init__(self, engine: Engine, npairs: int, nbuf: int = 3):

@@ -50,6 +50,23 @@ size_t ws_elems(const Engine& e) { return (size_t)(5 * e.k + 10 * e.kl) * e.N; }
 
 }  // namespace
 
+// Waits for the stream, then reads and clears the engine's error flag.
+int cpoly::sync_and_check(const Engine& e, const char* name, cudaStream_t st) {
+  int flag = 0;
+  cudaError_t err = cudaMemcpyAsync(&flag, e.d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
+  if (err == cudaSuccess) err = cudaStreamSynchronize(st);
+  if (err != cudaSuccess) return cuda_fail(name, err);
+  if (!flag) return CP_OK;
+  cudaMemsetAsync(e.d_err, 0, sizeof(int), st);
+  cudaStreamSynchronize(st);
+  std::string what;
+  if (flag & kErrSampler) what += ", sampler rejection limit reached";
+  if (flag & kErrWait) what += ", a wait inside a tensor-core kernel ran out: results since the last check are invalid";
+  if (flag & kErrTile) what += ", a work-list tile outside its group was skipped";
+  set_error("a kernel reported an error: " + (what.empty() ? "code " + std::to_string(flag) : what.substr(2)));
+  return CP_ERR_DEVICE;
+}
+
 extern "C" {
 
 const char* cp_version(void) { return "cupoly_b200 0.1.0 (sm_100a)"; }
@@ -363,21 +380,7 @@ size_t cp_workspace_bytes(const cp_engine* h) { return h ? ws_elems(h->e) * 16 :
 
 int cp_engine_check(const cp_engine* h, void* stream) {
   CP_REQUIRE(h, "cp_engine_check: NULL engine");
-  int flag = 0;
-  cudaError_t err = cudaMemcpyAsync(&flag, h->e.d_err, sizeof(int), cudaMemcpyDeviceToHost, S(stream));
-  if (err == cudaSuccess) err = cudaStreamSynchronize(S(stream));
-  if (err != cudaSuccess) return cuda_fail("cp_engine_check", err);
-  if (flag) {
-    cudaMemsetAsync(h->e.d_err, 0, sizeof(int), S(stream));
-    cudaStreamSynchronize(S(stream));
-    std::string what;
-    if (flag & kErrSampler) what += ", sampler rejection limit reached";
-    if (flag & kErrWait) what += ", a wait inside a tensor-core kernel ran out: results since the last check are invalid";
-    if (flag & kErrTile) what += ", a work-list tile outside its group was skipped";
-    set_error("a kernel reported an error: " + (what.empty() ? "code " + std::to_string(flag) : what.substr(2)));
-    return CP_ERR_DEVICE;
-  }
-  return CP_OK;
+  return sync_and_check(h->e, "cp_engine_check", S(stream));
 }
 
 int cp_engine_check_async(const cp_engine* h, int* flag_host, void* stream) {

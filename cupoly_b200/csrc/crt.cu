@@ -708,10 +708,9 @@ int cp_export_residues(const cp_engine* h, void* host_out, size_t cap, const voi
   std::memcpy(o + sizeof(hd), base_primes(e, base, tmp), (size_t)nres * 8);
   const size_t body = (size_t)npolys * nres * e.N * 16;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  cudaError_t err = cudaMemcpyAsync(o + sizeof(hd) + (size_t)nres * 8, poly, body, cudaMemcpyDeviceToHost, st);
-  if (err == cudaSuccess) err = cudaStreamSynchronize(st);
+  const cudaError_t err = cudaMemcpyAsync(o + sizeof(hd) + (size_t)nres * 8, poly, body, cudaMemcpyDeviceToHost, st);
   if (err != cudaSuccess) return cuda_fail("cp_export_residues", err);
-  return CP_OK;
+  return sync_and_check(e, "cp_export_residues", st);
 }
 
 int cp_import_residues(const cp_engine* h, void* poly, const void* host_in, size_t size, int base, int npolys,

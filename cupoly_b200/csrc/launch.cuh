@@ -42,6 +42,9 @@ inline int check_launch(const char* what) {
   return CP_OK_;
 }
 
+// Waits for the stream, then reads and clears the engine's error flag (capi.cu).
+int sync_and_check(const Engine& e, const char* name, cudaStream_t st);
+
 // Raise a kernel's dynamic shared-memory limit once per device.
 template <typename K>
 inline int ensure_smem(K kernel, int bytes, std::atomic<unsigned long long>& done_mask) {

@@ -254,7 +254,7 @@ def poly_icrt(ctx: Context, a: poly_t, x: torch.Tensor):
     with torch.cuda.stream(ctx.stream):
         limbs = torch.empty((1, 2 * CUDAEngine.N, nl), dtype=torch.int64, device="cuda")
     e.icrt(limbs, x, a.base, stream=ctx.stream)
-    ctx.stream.synchronize()
+    e.check(ctx.stream)  # waits; raises what a kernel has reported
     a.coefs = limbs_to_ints(to_u64(limbs[0]))
 
 
@@ -339,7 +339,7 @@ def poly_export_residues(ctx: Context, a: poly_t) -> str:
     with torch.cuda.stream(ctx.stream):
         aux = a.d_coefs.clone()
     e.dgt(aux, a.base, INVERSE, stream=ctx.stream)
-    ctx.stream.synchronize()
+    e.check(ctx.stream)
     h = e.unfold(to_u64(aux[0]))
     return " ".join(str(int(v)) for v in h.reshape(-1).astype(np.int64))
 

@@ -139,6 +139,7 @@ class Engine:
         self.Q = self.primes[: self.k]
         self.B = self.primes[self.k:]
         self._wsbuf: Optional[torch.Tensor] = None
+        self._flag: Optional[torch.Tensor] = None
         self.device = torch.cuda.current_device()
 
     # ---- DGT plan ----
@@ -263,6 +264,17 @@ class Engine:
     def check_async(self, flag_host: torch.Tensor, stream=None):
         """Queue a copy of the engine's error flag into flag_host (a pinned int32 tensor) on the stream."""
         call("cp_engine_check_async", self._h, _ptr(flag_host), _stream(stream))
+
+    def download(self, t: torch.Tensor) -> np.ndarray:
+        """Results of this engine to the host (to_u64 on the current stream); raises if a kernel has
+        reported an error."""
+        if self._flag is None:
+            self._flag = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self.check_async(self._flag)
+        out = to_u64(t)
+        if int(self._flag[0]):
+            self.check()
+        return out
 
     # ---- DGT ----
     def dgt(self, x: torch.Tensor, base: int, direction: int, npolys: Optional[int] = None, stream=None):

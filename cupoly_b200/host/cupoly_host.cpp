@@ -270,6 +270,8 @@ void d2d(void* dst, const void* src, size_t bytes, Context* ctx) {
 }
 
 void sync(Context* ctx) { cuda_check(cudaStreamSynchronize(ctx->get_stream()), "cudaStreamSynchronize"); }
+// Before results are handed to the host: waits, and throws what a kernel has reported.
+void sync_results(Context* ctx, const char* what) { check(cp_engine_check(E(), S(ctx)), what); }
 
 // Inputs to the device; output initialised for `base` (cuPoly's lazy poly_init of outputs).
 void prep_out(Context* ctx, poly_t* out, int base) {
@@ -562,7 +564,7 @@ void poly_icrt(Context* ctx, poly_t* a) {
   uint64_t* h = ctx->host_scratch((size_t)n * nl);
   cuda_check(cudaMemcpyAsync(h, d, (size_t)n * nl * 8, cudaMemcpyDeviceToHost, ctx->get_stream()),
              "cudaMemcpyAsync");
-  sync(ctx);
+  sync_results(ctx, "poly_icrt");
   a->coefs.resize(n);
   for (int i = 0; i < n; ++i) a->coefs[i] = zz_from_limbs(h + (size_t)i * nl, nl);
 }
@@ -944,7 +946,7 @@ static void host_residues(Context* ctx, poly_t* a, std::vector<uint64_t>& out) {
   std::vector<GaussianInteger> h((size_t)nr * N);
   cuda_check(cudaMemcpyAsync(h.data(), aux, res_bytes(a->base), cudaMemcpyDeviceToHost, ctx->get_stream()),
              "cudaMemcpyAsync");
-  sync(ctx);
+  sync_results(ctx, "residue access");
   out.assign((size_t)nr * 2 * N, 0);
   for (int r = 0; r < nr; ++r)
     for (int j = 0; j < N; ++j) {

@@ -148,7 +148,8 @@ size_t cp_workspace_bytes(const cp_engine* e);
  *     reads or writes integer coefficients: cp_dgt*, cp_polymul*, cp_sample* with to_dgt, cp_bfv_mul*,
  *     cp_crt, cp_icrt and the composites): a wait for a copy or a product ran out after about
  *     2 s on the device.  It cannot happen in a working program; if it does, the results written since the
- *     last check are invalid. */
+ *     last check are invalid.
+ * cp_export_residues makes this check before it returns. */
 int cp_engine_check(const cp_engine* e, void* stream);
 /* the engine's error flag, copied into flag_host (page-locked host memory) on `stream` behind
  * the work already queued there, without waiting: nonzero once the copy has completed means
