@@ -241,8 +241,19 @@ int cp_engine_set_tensor(cp_engine* h, int mode) {
   CP_REQUIRE(h, "cp_engine_set_tensor: NULL engine");
   CP_REQUIRE(mode >= 0 && mode <= 2, "cp_engine_set_tensor: mode must be 0, 1 or 2");
   Engine& e = h->e;
+  if (mode == 2 && !tensor_possible(e)) {
+    set_error("cp_engine_set_tensor: no tensor-core transforms for this engine (a BFV engine of nphi 2048 .. 65536; "
+              "from 32768 on with 2 split bits in its plan)");
+    return CP_ERR_UNSUPPORTED;
+  }
   cudaDeviceSynchronize();
   e.tensor = mode;
+  e.narrow_first = 0;
+  e.cluster_first = false;
+  if ((mode != 0 && tensor_possible(e)) == (e.d_ttab != nullptr)) {  // the tables are there, or are not needed
+    place_tensor_line(e);
+    return CP_OK;
+  }
   free_tables(e);
   return build_tables_nothrow(e);
 }
@@ -270,6 +281,7 @@ int cp_engine_set_narrow_plan(cp_engine* h, int log_radix, int log_cta, long lon
     e.plan_narrow = DgtPlan{};
   }
   e.narrow_units = max_units;
+  e.narrow_first = max_units;
   return build_tables_nothrow(e);
 }
 
@@ -287,7 +299,14 @@ int cp_engine_set_split_mode(cp_engine* h, int mode) {
   CP_REQUIRE(mode == 0 || mode == 1, "cp_engine_set_split_mode: mode must be 0 (split kernel) or 1 (cluster)");
   cudaDeviceSynchronize();  // transforms in flight keep the form they were launched with
   h->e.plan.cluster = mode;
+  h->e.cluster_first = mode == 1;
   return CP_OK;
+}
+
+int cp_engine_dgt_launches(const cp_engine* h, long long units, int work_list, int* on_tensor) {
+  if (!h || units < 0) return -1;
+  if (on_tensor) *on_tensor = units > 0 && dgt_on_tensor(h->e, units, work_list != 0) ? 1 : 0;
+  return dgt_launches(h->e, units, work_list != 0);
 }
 
 int cp_engine_get_split_mode(const cp_engine* h) { return h ? h->e.plan.cluster : -1; }

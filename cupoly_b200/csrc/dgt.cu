@@ -270,7 +270,17 @@ int run_transform(const Engine& e, ulonglong2* data, const FwdIO& fio, const Inv
 }  // namespace
 
 bool dgt_on_tensor(const Engine& e, long long units, bool list) {
-  return e.d_ttab && !(list && e.tlayout.S > 0) && units > e.tensor_above;
+  if (!e.d_ttab || (list && e.tlayout.S > 0)) return false;
+  if (e.tensor == 1 && (units <= e.narrow_first || (e.cluster_first && e.plan.S > 0))) return false;
+  return units > e.tensor_above;
+}
+
+int dgt_launches(const Engine& e, long long units, bool list) {
+  if (units <= 0) return 0;
+  if (dgt_on_tensor(e, units, list))
+    return list ? (int)((units + kTdgtListMax - 1) / kTdgtListMax) : (e.tlayout.S > 0 ? 2 : 1);
+  const DgtPlan& P = select_plan(e, units).P;
+  return P.S == 0 || (P.cluster && pick_cluster(P.logNc, P.logR, P.S)) ? 1 : 2;
 }
 
 int launch_dgt_ex(const Engine& e, void* dst_v, const void* fsrc_v, const InvSrc* isrc_p, int base, int npolys,

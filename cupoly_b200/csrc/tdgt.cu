@@ -53,7 +53,6 @@ using namespace umma;
 
 constexpr int kEpiWarps = 16;
 constexpr int kThreads = (kEpiWarps + 1) * 32;
-constexpr int kListMax = 4096;  // rows of a work list per launch (their order lives in shared memory)
 
 struct TArgs {
   const uint8_t* tab;  // table block of residue 0
@@ -448,7 +447,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ uint32_t s_slot;
   __shared__ int s_fail;
   __shared__ unsigned s_cnt[kMaxResidues + 1], s_ustart[kMaxResidues + 1];
-  __shared__ uint16_t s_order[kListMax];
+  __shared__ uint16_t s_order[kTdgtListMax];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t sdat = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sB1 = sdat + C::DATA;
@@ -970,8 +969,8 @@ int launch_tdgt(const Engine& e, ulonglong2* data, const ulonglong2* fsrc, const
     A.nunits = (unsigned)(per * nres);
     return launch_any(M, inverse, A, A.nunits, st);
   }
-  for (int i0 = 0; i0 < npolys; i0 += kListMax) {  // rows of the list, kListMax at a time
-    const int n = npolys - i0 < kListMax ? npolys - i0 : kListMax;
+  for (int i0 = 0; i0 < npolys; i0 += kTdgtListMax) {  // rows of the list, kTdgtListMax at a time
+    const int n = npolys - i0 < kTdgtListMax ? npolys - i0 : kTdgtListMax;
     const size_t o = (size_t)i0 * poly_stride;
     TArgs B = A;
     B.rid_list = rid_list + i0;

@@ -4,6 +4,8 @@
 
 namespace cpoly {
 
+constexpr int kTdgtListMax = 4096;  // rows of a work list per launch (their order lives in shared memory)
+
 // One transform of npolys x nres residues (see run_transform in dgt.cu), the element blocks of
 // 2^tlayout.logNc elements on the tensor cores.  With tlayout.S > 0 the blocks are the 2^S
 // parts that the split stage leaves, without a twist.

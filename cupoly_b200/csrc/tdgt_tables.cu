@@ -133,19 +133,28 @@ void build_residue(const Engine& e, int r, uint64_t pre0, uint64_t pre1, uint8_t
 
 }  // namespace
 
-// Places and fills the tensor-core tables when the engine can use them: 63-bit primes (the
-// kernels reduce by 2^63 = c), blocks of 2^10 .. 2^13 elements, at most the default 2 split bits.
-int build_tensor_tables(Engine& e) {
-  e.tlayout = TdgtLayout{};
-  const int logNc = e.logN <= 13 ? e.logN : e.logN - 2;
-  if (!e.tensor || e.ckks_prec || logNc < 10 || (e.logN > 13 && (e.plan.S != 2 || e.plan.logNc != logNc))) return 0;
+// 63-bit primes (the kernels reduce by 2^63 = c), blocks of 2^10 .. 2^13 elements; above, the main
+// plan's split stage does the default 2 bits.
+bool tensor_possible(const Engine& e) {
+  return !e.ckks_prec && e.logN >= 10 && (e.logN <= 13 || (e.plan.S == 2 && e.plan.logNc == e.logN - 2));
+}
+
+void place_tensor_line(Engine& e) {
   // Launches of at most this many residue transforms keep the CUDA-core plans, whose small
   // launches spread one residue over several CTAs: a tensor-core unit takes 11 us however few
   // there are (22 us at N = 8192).  Forward + inverse at the line, us, CUDA cores / tensor cores:
   // nphi 2048: 288 residues 19 / 24, 384 25 / 24; 4096: 64 18 / 23, 96 22 / 23, 148 24 / 23;
   // 8192: 32 19 / 24, 64 24 / 24; 16384: 32 28 / 44, 64 43 / 44; 32768: 1 36 / 31.
   static const int above[5] = {320, 96, 64, 64, 0};
-  e.tensor_above = e.tensor == 2 ? 0 : above[e.logN - 10 < 4 ? e.logN - 10 : 4];
+  e.tensor_above = e.tensor == 2 ? 0 : above[e.logN < 10 ? 0 : (e.logN < 14 ? e.logN - 10 : 4)];
+}
+
+// Places and fills the tensor-core tables when the engine can use them.
+int build_tensor_tables(Engine& e) {
+  e.tlayout = TdgtLayout{};
+  if (!e.tensor || !tensor_possible(e)) return 0;
+  place_tensor_line(e);
+  const int logNc = e.logN <= 13 ? e.logN : e.logN - 2;
   TdgtLayout& L = e.tlayout;
   L.logNc = logNc;
   L.S = e.logN - logNc;

@@ -10,7 +10,7 @@ used only for device memory and streams; every computation is a call into
 from __future__ import annotations
 
 import ctypes as C
-from typing import List, Optional, Sequence
+from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
 import torch
@@ -121,12 +121,13 @@ class Engine:
         logN = (nphi // 2).bit_length() - 1
         if tuned_radix and (plan["log_radix"], plan["log_cta"]) != (min(tuned_radix, logN), min(log_cta or 13, logN)):
             call("cp_engine_set_plan", h, tuned_radix, log_cta)
-            call("cp_engine_set_tensor", h, 1)  # the tuned CUDA-core plan serves what the tensor cores do not
         if split_mode:
             call("cp_engine_set_split_mode", h, split_mode)
         if narrow is not None and narrow != (small["log_radix"], small["log_cta"], small["max_units"]) and \
                 (narrow[2] or small["max_units"]):
             call("cp_engine_set_narrow_plan", h, narrow[0], narrow[1], narrow[2])
+        if log_radix == 0:
+            call("cp_engine_set_tensor", h, 1)  # the tuned CUDA-core plans serve what the tensor cores do not
         self.log_radix = log_radix or tuned_radix
         self.k = k
         self.kl = kl if kl > 0 else k + 1
@@ -150,11 +151,19 @@ class Engine:
 
     def set_tensor(self, mode: int):
         """Transforms on the tensor cores in launches large enough to gain (1, the default), in
-        every launch (2) or never (0); same results.  set_plan selects 0; rebuilds the tables."""
+        every launch (2) or never (0); same results.  Of this and the plan settings the later call goes
+        first (see cp_engine_set_tensor)."""
         call("cp_engine_set_tensor", self._h, int(mode))
 
     def get_tensor(self) -> bool:
         return _lib.lib().cp_engine_get_tensor(self._h) == 1
+
+    def dgt_launches(self, units: int, work_list: bool = False) -> Tuple[int, bool]:
+        """Kernels of one transform launch of `units` residue transforms, and whether they are the
+        tensor-core ones (where the products of a fused call are a kernel of their own)."""
+        t = C.c_int()
+        n = _lib.lib().cp_engine_dgt_launches(self._h, int(units), 1 if work_list else 0, C.byref(t))
+        return n, t.value == 1
 
     def set_split_mode(self, mode: int):
         """0: split stage as its own kernel (HBM pass); 1: inside a thread-block cluster (DSMEM)."""

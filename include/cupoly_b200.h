@@ -95,11 +95,20 @@ int cp_engine_set_plan(cp_engine* e, int log_radix, int log_cta);
 
 /* Transforms on the tensor cores (BFV engines, nphi 2048 .. 65536; results are identical): 1, the
  * default of an engine created with log_radix 0: in launches large enough to gain from them;
- * 2: in every launch; 0: never.  cp_engine_set_plan selects 0.  Rebuilds the engine's tables
+ * 2: in every launch (CP_ERR_UNSUPPORTED where the engine has no such transforms: CKKS, other
+ * degrees, or from nphi 32768 on a plan without 2 split bits); 0: never.  Of this and the plan settings below the
+ * later call goes first: cp_engine_set_plan selects 0; in mode 1 a launch of at most
+ * cp_engine_set_narrow_plan's max_units runs with that plan, and with cp_engine_set_split_mode 1 a
+ * transform larger than one CTA runs in its cluster; a further call of this returns them to the tensor
+ * cores.  In mode 2 no plan setting but cp_engine_set_plan matters.  Rebuilds the engine's tables when they change
  * (synchronises the device). */
 int cp_engine_set_tensor(cp_engine* e, int mode);
 /* 1: the engine holds tensor-core tables; 0: it does not; -1: NULL engine. */
 int cp_engine_get_tensor(const cp_engine* e);
+/* Kernels that one transform launch of `units` residue transforms (polynomials x residues; work_list:
+ * rows of a list) takes with the present settings; -1: NULL engine or units < 0.  *on_tensor (may be NULL): 1 when
+ * they are the tensor-core ones, where the products of a fused call are a kernel of their own. */
+int cp_engine_dgt_launches(const cp_engine* e, long long units, int work_list, int* on_tensor);
 int cp_engine_get_plan(const cp_engine* e, int* log_radix, int* log_cta, int* split_bits);
 /* Second DGT plan for small launches (no counterpart in cuPoly): a transform launch of at
  * most max_units residue transforms (polynomials x residues) uses (log_radix, log_cta)
