@@ -215,7 +215,8 @@ namespace {
 // then the split stage.  With the cluster form the split stage runs inside the kernel.
 int run_transform(const Engine& e, ulonglong2* data, const FwdIO& fio, const InvSrc& isrc, int nres,
                   int rid_off, int npolys, long long poly_stride, bool inverse, cudaStream_t st, const int* rid_list) {
-  if (dgt_on_tensor(e, (long long)npolys * nres, rid_list != nullptr)) {
+  // the tensor-core kernel has one source and one output
+  if (!fio.scatter[0] && !fio.src_polys && dgt_on_tensor(e, (long long)npolys * nres, rid_list != nullptr)) {
     if (inverse && isrc.untwist > 2) {
       set_error("dgt: unknown untwist table");
       return 1;
@@ -320,7 +321,7 @@ int launch_dgt_pair(const Engine& e, void* dst_v, const void* a_v, const void* b
   ulonglong2* dst = reinterpret_cast<ulonglong2*>(dst_v);
   const ulonglong2 *a = reinterpret_cast<const ulonglong2*>(a_v), *b = reinterpret_cast<const ulonglong2*>(b_v);
   const bool same_plan = &select_plan(e, units).P == &select_plan(e, 2 * units).P;
-  // (the tensor-core kernel has one source; a grid for both must not be refused where one was accepted)
+  // (large calls run on the tensor cores; a grid for both must not be refused where one was accepted)
   if (dgt_on_tensor(e, 2 * units) || !same_plan || 2 * units * (e.N / 256 + 1) > 0x7fffffffLL) {
     if (int rc = launch_dgt_ex(e, dst, a, nullptr, base, npolys, 0, false, st)) return rc;
     return launch_dgt_ex(e, dst + npolys * stride, b, nullptr, base, npolys, 0, false, st);
@@ -330,6 +331,8 @@ int launch_dgt_pair(const Engine& e, void* dst_v, const void* a_v, const void* b
   return run_transform(e, dst, fio, InvSrc{}, nres, e.rid_offset(base), 2 * npolys, stride, false, st, nullptr);
 }
 
+// One launch for the three, on the CUDA cores, unless each of them is large enough for the tensor
+// cores by itself (from nphi 32768 on always: 31 against 36 us for one residue).
 int launch_dgt_scatter3(const Engine& e, void* const dst[3], const void* src_v, int base, cudaStream_t st) {
   const int nres = e.n_residues(base);
   if (nres < 0 || base == 3) {
@@ -338,7 +341,7 @@ int launch_dgt_scatter3(const Engine& e, void* const dst[3], const void* src_v, 
   }
   const ulonglong2* src = reinterpret_cast<const ulonglong2*>(src_v);
   const long long stride = (long long)nres * e.N;
-  if (dgt_on_tensor(e, 3LL * nres)) {  // the tensor-core kernel has one output
+  if (dgt_on_tensor(e, nres)) {
     for (int v = 0; v < 3; ++v)
       if (int rc = launch_dgt_ex(e, dst[v], src + v * stride, nullptr, base, 1, 0, false, st)) return rc;
     return 0;
