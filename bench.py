@@ -518,9 +518,9 @@ def run_ours(args, D: Dist):
     ms = D.max(ev0.elapsed_time(ev1))
     value = D.world * P * args.steps / (ms / 1e3)
     # inverse DGT (gather) + Q->B + forward DGT(B) + 2 inverse DGTs of the tensor product + complex
-    # scaling + B->Q + forward DGT(Q) (nphi <= 16384: one kernel per DGT); the products are two
-    # kernels of their own on the tensor cores, part of the inverses on the CUDA cores
-    launches_per_step = 10 if e.get_tensor() else 8
+    # scaling + B->Q + forward DGT(Q); the products are two kernels of their own on the tensor
+    # cores, part of the inverses on the CUDA cores
+    launches_per_step = e.bfv_mul_batch_launches(P)
 
     # ---- e2e: host-resident batches through the public API (StreamedBFV: copy-in,
     # chain and copy-out of consecutive batches overlap on three streams); every
@@ -730,7 +730,6 @@ def run_ours(args, D: Dist):
              "form": {"sequence": "one CUDA graph, per size group a fused cp_polymul_list (3 launches; 4 on the tensor cores)",
                       "branches": "the same graph with one parallel branch per size group",
                       "tiles": "one persistent launch (cp_polymul_tiles) over a work list of tiles"}[best],
-             # transform launches; on the tensor cores the products are one more per size group
              "launches_per_batch": mixed_launches[best],
              "polymul_per_s": round(1024 / (mixed_ms / 1e3), 1), "ms_per_batch": round(mixed_ms, 3),
              "ms_per_batch_by_form": {k_: round(v_, 4) for k_, v_ in mixed_forms.items()},

@@ -42,7 +42,7 @@ class MixedPolymul:
                  mode: str = "graph"):
         """specs[i] = (nphi_i, k_i) with 1 <= k_i <= kmax.
 
-        mode "graph": per size group one fused cp_polymul_list (3 launches) with the
+        mode "graph": per size group one fused cp_polymul_list (see launches_per_run) with the
         group engine's tuned plan, all captured in one CUDA graph (see capture);
         mode "tiles": the whole batch in ONE persistent launch (cp_polymul_tiles) over
         a device work list of same-size tiles; every size must be in TILE_SIZES."""
@@ -137,7 +137,7 @@ class MixedPolymul:
 
     # ---- execution ----
     def _launch_group(self, g, stream):
-        # fused: 2 out-of-place forward DGTs, inverse with products on load
+        # fused: 2 out-of-place forward DGTs, the products (on load or by themselves), the inverse
         e, n, rid = g["engine"], g["rows"], g["rid"]
         call("cp_polymul_list", e.handle, _ptr(g["c"]), _ptr(g["a"]), _ptr(g["b"]), _ptr(g["wa"]),
              _ptr(g["wb"]), _ptr(rid), n, _stream(stream))
@@ -192,9 +192,12 @@ class MixedPolymul:
         self.graph.replay()
 
     def launches_per_run(self) -> int:
-        """Transform launches of one run, with the products in the inverse; a group large enough for the
-        tensor cores takes one more, its products."""
-        return 1 if self.mode == "tiles" else 3 * len(self.groups)
+        """Launches of one run: per size group two forward transforms and an inverse (each counted as one,
+        whatever kernels its plan takes), and the products where the group runs on the tensor
+        cores."""
+        if self.mode == "tiles":
+            return 1
+        return sum(3 + int(g["engine"].dgt_launches(g["rows"], work_list=True)[1]) for g in self.groups.values())
 
     def algorithmic_bytes(self) -> int:
         """24 nphi k bytes per product: read a, b and write c (16 B per Gaussian element)."""

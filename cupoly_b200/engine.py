@@ -165,6 +165,14 @@ class Engine:
         n = _lib.lib().cp_engine_dgt_launches(self._h, int(units), 1 if work_list else 0, C.byref(t))
         return n, t.value == 1
 
+    def bfv_mul_batch_launches(self, npairs: int) -> int:
+        """Kernels of one bfv_mul_batch call: three base conversions, the transforms of 4 npairs inputs over
+        Q and over B and of 3 npairs outputs over Q, over B and over Q again, and the products over a
+        base whose inverse runs on the tensor cores."""
+        q, b = npairs * self.k, npairs * self.kl
+        n = 3 + sum(self.dgt_launches(u)[0] for u in (4 * q, 4 * b, 3 * q, 3 * b, 3 * q))
+        return n + sum(int(self.dgt_launches(u)[1]) for u in (3 * q, 3 * b))
+
     def set_split_mode(self, mode: int):
         """0: split stage as its own kernel (HBM pass); 1: inside a thread-block cluster (DSMEM)."""
         call("cp_engine_set_split_mode", self._h, int(mode))
