@@ -139,6 +139,7 @@ cp_engine* new_engine(int k, int kl, int nphi, uint64_t t) {
   }
   Engine& e = h->e;
   cudaGetDevice(&e.device);
+  if (cudaDeviceGetAttribute(&e.sms, cudaDevAttrMultiProcessorCount, e.device) != cudaSuccess || e.sms < 1) e.sms = 1;
   e.k = k;
   e.kl = kl;
   e.nphi = nphi;

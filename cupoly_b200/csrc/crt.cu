@@ -467,12 +467,9 @@ IcrtTensorFn icrt_tensor_kernel(int ns, std::integer_sequence<int, I...>) {
   return table[ns - kIcrtFirst];
 }
 
-int io_ctas(int smem_bytes, int most_per_sm) {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+int io_ctas(const Engine& e, int smem_bytes, int most_per_sm) {
   const int fit = 220 * 1024 / (smem_bytes + 1024);
-  return (sms > 0 ? sms : 1) * std::max(1, std::min(fit, most_per_sm));
+  return e.sms * std::max(1, std::min(fit, most_per_sm));
 }
 
 __global__ void __launch_bounds__(256) k_icrt_t(uint64_t* __restrict__ coefs, int nlimbs,
@@ -619,7 +616,7 @@ int cp_crt(const cp_engine* h, void* out, const uint64_t* coefs, int nlimbs, int
       static std::atomic<unsigned long long> done{0};
       if (int rc = ensure_smem(k_crt_tensor, 200 * 1024, done)) return rc;
       const IoTensor io{e.d_io, e.io_cols, e.N / 128, (int)tiles, inv_small(nlimbs), e.d_err};
-      k_crt_tensor<<<(unsigned)std::min<long long>(tiles, io_ctas(smem, 4)), 128, smem,
+      k_crt_tensor<<<(unsigned)std::min<long long>(tiles, io_ctas(e, smem, 4)), 128, smem,
                      reinterpret_cast<cudaStream_t>(stream)>>>(reinterpret_cast<ulonglong2*>(out), coefs, nlimbs, e.N,
                                                                nres, e.rid_offset(base), e.d_mc, io);
       return check_launch("cp_crt");
@@ -629,9 +626,10 @@ int cp_crt(const cp_engine* h, void* out, const uint64_t* coefs, int nlimbs, int
   const int T = nlimbs <= 23 ? 128 : (nlimbs <= 47 ? 64 : 32);
   const unsigned bx = (unsigned)((e.N + T - 1) / T), groups = (unsigned)((nres + 3) / 4);
   // The blocks of a small call take one group of residues each (a group's serial chain is the
-  // whole time); with four blocks on each of 148 SMs reading the limbs once is worth more.
+  // whole time); with four blocks on each SM reading the limbs once is worth more.
   const long long blocks = (long long)bx * npolys;
-  const unsigned gz = blocks >= 592 ? 1u : (unsigned)std::min<long long>(groups, (592 + blocks - 1) / blocks);
+  const long long fill = 4LL * e.sms;
+  const unsigned gz = blocks >= fill ? 1u : (unsigned)std::min<long long>(groups, (fill + blocks - 1) / blocks);
   k_crt<<<dim3(bx, (unsigned)npolys, gz), T, (size_t)2 * T * (nlimbs | 1) * 8, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<ulonglong2*>(out), coefs, nlimbs, e.N, nres, e.rid_offset(base), e.d_mc, e.d_hps + e.ho.pow64,
       e.d_hps + e.ho.pow64m, inv_small(nlimbs), e.ckks_prec ? 0 : 1);
@@ -666,7 +664,7 @@ int cp_icrt(const cp_engine* h, uint64_t* coefs, int nlimbs, const void* in, int
       static std::atomic<unsigned long long> done[kIcrtTensor + 1];
       if (int rc = ensure_smem(fn, smem, done[ns])) return rc;
       const IoTensor io{e.d_io + e.io_icrt[base == CP_QBASE ? 0 : 1], 0, e.N / 128, (int)tiles, inv_small(nlimbs), e.d_err};
-      fn<<<(unsigned)std::min<long long>(tiles, io_ctas(smem, per)), 128, smem, st>>>(coefs, nlimbs, src, e.N,
+      fn<<<(unsigned)std::min<long long>(tiles, io_ctas(e, smem, per)), 128, smem, st>>>(coefs, nlimbs, src, e.N,
                                                                                       e.rid_offset(base), e.d_mc, io);
       return check_launch("cp_icrt");
     }

@@ -116,6 +116,7 @@ struct MrcTables {
 
 struct Engine {
   int device = 0;
+  int sms = 1;  // multiprocessors of the device
   int nphi = 0, N = 0, logN = 0;
   int k = 0, kl = 0;
   uint64_t t = 0;

@@ -875,16 +875,13 @@ int launch_conv_tensor(const Engine& e, int which, ulonglong2* out, const ulongl
   int smem = 2 * 128 * sh.kbytes() + sh.bytes();
   if (smem < 46 * 1024) smem = 46 * 1024;  // at most four CTAs a SM: each holds 128 columns of tensor memory
   if (int rc = ensure_smem(k_conv_tensor<NS, SCALE, Args>, 2 * 128 * 224 + 224 * 192, done)) return rc;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = (long long)npolys * (e.N / 128);
   if (tiles > 0x3fffffffLL) {
     set_error("base conversion: batch too large");
     return CP_ERR_INVALID_;
   }
   const int per = smem <= 56 * 1024 ? 4 : (smem <= 75 * 1024 ? 3 : 2);
-  const long long most = (long long)(sms > 0 ? sms : 1) * per;
+  const long long most = (long long)e.sms * per;
   const TensorConv tc{e.d_cmat + e.cmat_off[which], e.N / 128, (int)tiles, e.d_err};
   k_conv_tensor<NS, SCALE, Args><<<(unsigned)(tiles < most ? tiles : most), 128, smem, st>>>(out, in, in_b, a, tc);
   return check_launch("base conversion (tensor cores)");

@@ -283,6 +283,10 @@ __global__ void __launch_bounds__(256)
 // this one's products are formed.  With one element per thread the loads of four terms were in
 // flight at a time, behind the prime's constants, and a block lived for one such chain: 44 us for
 // 64 polynomials of 5 terms at nphi 8192, k 5 (20 us of traffic), 25.5 us so.
+// A term takes 12 registers.  The line of 8 terms is how far the kernel was taken (8 terms, nphi 8192,
+// 40 polynomials: 57.0 us with one element per thread, 45.3 us so), not where it stops gaining: with the
+// table below extended, 9 terms of 32 polynomials took 57.1 and 44.3 us, 16 terms at nphi 32768 of 4
+// polynomials 94 and 69 us.
 constexpr int kDotHeld = 8;
 template <int NT>
 __global__ void __launch_bounds__(128)
@@ -405,10 +409,10 @@ int pw_dot_batch(const Engine& e, void* c, const void* a, const void* b, int n, 
     static constexpr Fn table[kDotHeld] = {k_dot_shared<1>, k_dot_shared<2>, k_dot_shared<3>, k_dot_shared<4>,
                                            k_dot_shared<5>, k_dot_shared<6>, k_dot_shared<7>, k_dot_shared<8>};
     const int bx = (e.N + 127) / 128;
-    // twelve blocks for each of 148 SMs (with 6 and 12 of them the above takes 25.5 us, with 20 26,
+    // twelve blocks for each SM (with 6 and 12 of them the above takes 25.5 us, with 20 26,
     // with 40 29: each starts with a load of b), each with a run of polynomials
     const long long rows = (long long)bx * nres;
-    long long runs = (148LL * 12 + rows - 1) / rows;
+    long long runs = (12LL * e.sms + rows - 1) / rows;
     if (runs > npolys) runs = npolys;
     table[n - 1]<<<dim3(bx, nres, (unsigned)runs), 128, 0, st>>>(CU2(a), CU2(b), U2(c), e.N, nres, e.rid_offset(base),
                                                                npolys, e.d_mc);

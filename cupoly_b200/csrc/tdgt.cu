@@ -37,6 +37,7 @@
 // products and the bulk copies.
 #include <cuda.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "byte_sums.cuh"
@@ -900,31 +901,27 @@ int forward_map(const TArgs& A, CUtensorMap* map) {
 }
 
 template <int M, bool INV>
-int launch_m(const TArgs& A, unsigned max_units, cudaStream_t st) {
+int launch_m(const TArgs& A, unsigned grid, cudaStream_t st) {
   CUtensorMap fmap{};
   if (!INV)
     if (int rc = forward_map<M>(A, &fmap)) return rc;
   static std::atomic<unsigned long long> done{0};
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   constexpr int smem = Cfg<M>::SMEM;
   if (int rc = ensure_smem(k_tdgt<M, INV>, smem, done)) return rc;
-  const unsigned grid = max_units < (unsigned)sms ? max_units : (unsigned)sms;
   k_tdgt<M, INV><<<grid, kThreads, smem, st>>>(A, fmap);
   return check_launch("dgt (tensor cores)");
 }
 
-int launch_any(int M, bool inv, const TArgs& A, unsigned max_units, cudaStream_t st) {
+int launch_any(int M, bool inv, const TArgs& A, unsigned grid, cudaStream_t st) {
   switch (M * 2 + (inv ? 1 : 0)) {
-    case 4: return launch_m<2, false>(A, max_units, st);
-    case 5: return launch_m<2, true>(A, max_units, st);
-    case 6: return launch_m<3, false>(A, max_units, st);
-    case 7: return launch_m<3, true>(A, max_units, st);
-    case 8: return launch_m<4, false>(A, max_units, st);
-    case 9: return launch_m<4, true>(A, max_units, st);
-    case 10: return launch_m<5, false>(A, max_units, st);
-    case 11: return launch_m<5, true>(A, max_units, st);
+    case 4: return launch_m<2, false>(A, grid, st);
+    case 5: return launch_m<2, true>(A, grid, st);
+    case 6: return launch_m<3, false>(A, grid, st);
+    case 7: return launch_m<3, true>(A, grid, st);
+    case 8: return launch_m<4, false>(A, grid, st);
+    case 9: return launch_m<4, true>(A, grid, st);
+    case 10: return launch_m<5, false>(A, grid, st);
+    case 11: return launch_m<5, true>(A, grid, st);
   }
   set_error("dgt (tensor cores): no kernel for this size");
   return CP_ERR_UNSUPPORTED_;
@@ -967,7 +964,7 @@ int launch_tdgt(const Engine& e, ulonglong2* data, const ulonglong2* fsrc, const
     }
     A.units_per_prime = (unsigned)per;
     A.nunits = (unsigned)(per * nres);
-    return launch_any(M, inverse, A, A.nunits, st);
+    return launch_any(M, inverse, A, std::min(A.nunits, (unsigned)e.sms), st);
   }
   for (int i0 = 0; i0 < npolys; i0 += kTdgtListMax) {  // rows of the list, kTdgtListMax at a time
     const int n = npolys - i0 < kTdgtListMax ? npolys - i0 : kTdgtListMax;
@@ -980,7 +977,7 @@ int launch_tdgt(const Engine& e, ulonglong2* data, const ulonglong2* fsrc, const
     B.data = data + o;
     B.fsrc = A.fsrc + o;
     for (int v = 0; v < 4; ++v) B.isrc.p[v] = isrc.p[v] ? isrc.p[v] + o : nullptr;
-    if (int rc = launch_any(M, inverse, B, (unsigned)n, st)) return rc;
+    if (int rc = launch_any(M, inverse, B, std::min((unsigned)n, (unsigned)e.sms), st)) return rc;
   }
   return 0;
 }
