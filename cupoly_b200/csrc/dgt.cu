@@ -72,7 +72,8 @@ int run_cta(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglon
   return check_launch("dgt");
 }
 
-using RunFn = int (*)(const Engine&, const DgtPlan&, const DgtTableLayout&, ulonglong2*, const FwdIO&, const InvSrc&, int, int, int, long long, bool, bool, cudaStream_t, const int*);
+using RunFn = int (*)(const Engine&, const DgtPlan&, const DgtTableLayout&, ulonglong2*, const FwdIO&, const InvSrc&,
+                      int, int, int, long long, bool, bool, cudaStream_t, const int*);
 
 constexpr int kNoCluster = -1;  // the cluster form cannot be scheduled on this device: use the split kernel
 

@@ -236,6 +236,8 @@ const char* last_error();
 
 // table construction (tables.cu)
 int build_tables(Engine& e);
+void prescale_factors(const Engine& e, std::vector<uint64_t>& pre0, std::vector<uint64_t>& pre1);
+void parallel_for_host(int n, void (*f)(int, void*), void* arg);  // f(i, arg) for i in [0, n) on the host's threads
 int build_io_tables(Engine& e);      // crt.cu
 int build_tensor_tables(Engine& e);  // tdgt_tables.cu; after the plans are placed
 bool tensor_possible(const Engine& e);  // whether those tables can be built beside the present plan

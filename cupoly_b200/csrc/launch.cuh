@@ -64,9 +64,10 @@ inline int ensure_smem(K kernel, int bytes, std::atomic<unsigned long long>& don
 // Kernel entry points implemented in the .cu files.
 int launch_dgt(const Engine& e, void* data, int base, int npolys, long long poly_stride, bool inverse,
                cudaStream_t st);
+// Forward transforms of npolys polynomials at a and of npolys at b into dst, one after the other.
+int launch_dgt_pair(const Engine& e, void* dst, const void* a, const void* b, int base, int npolys, cudaStream_t st);
 // Out-of-place forms: forward reads `fsrc` (nullptr = in place); inverse reads
 // per `isrc` (nullptr = in place).  Output always to `dst`.
-int launch_dgt_pair(const Engine& e, void* dst, const void* a, const void* b, int base, int npolys, cudaStream_t st);
 int launch_dgt_ex(const Engine& e, void* dst, const void* fsrc, const InvSrc* isrc, int base, int npolys,
                   long long poly_stride, bool inverse, cudaStream_t st);
 // Whether a launch of `units` residue transforms runs on the tensor cores.

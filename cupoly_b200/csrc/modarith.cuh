@@ -84,24 +84,8 @@ CP_HD void mac192_w(uint64_t& l, uint64_t& h, uint64_t& t, uint64_t a, uint64_t 
 
 // (t 2^128 + h 2^64 + l) mod p for t < 2^8, using r1 = 2^64 mod p < 2^32 and
 // r2 = 2^128 mod p: fold the high words down three times, then at most two
-// subtractions (the value is below 2^64 < 3p).
-CP_HD uint64_t red192(uint64_t l, uint64_t h, uint64_t t, uint64_t p, uint64_t r1, uint64_t r2) {
-  const uint32_t r = (uint32_t)r1;  // r1 < 2^32: 64 x 32-bit products below
-  // y = l + h r1 + t r2 < 2^97
-  unsigned __int128 y = (unsigned __int128)l + (unsigned __int128)h * r + (unsigned __int128)t * r2;
-  // z = lo(y) + hi(y) r1 < 2^66
-  unsigned __int128 z = (unsigned __int128)(uint64_t)y + (unsigned __int128)(uint64_t)(y >> 64) * r;
-  // w = lo(z) + hi(z) r1 < 2^64 + 2^34; one carry at most
-  const uint64_t zl = (uint64_t)z, zh = (uint64_t)(z >> 64);
-  uint64_t w = zl + zh * r1;
-  if (w < zl) w += r1;
-  w = w >= p ? w - p : w;
-  w = w >= p ? w - p : w;
-  return w;
-}
-
-// red192 with every product written as 32 x 32 -> 64 multiplies (r1 < 2^32, t < 2^8):
-// seven wide multiplies; used by the base conversions.
+// subtractions (the value is below 2^64 < 3p).  Every product is written as 32 x 32 -> 64
+// multiplies, seven of them; used by the base conversions.
 CP_HD uint64_t red192_w(uint64_t l, uint64_t h, uint64_t t, uint64_t p, uint64_t r1, uint64_t r2) {
   const uint64_t r = (uint32_t)r1;
   // y = l + h r1 + t r2 < 2^97

@@ -194,12 +194,11 @@ struct DoubleOpIntF {
 // c = sum_t a_t b_t (+ c when `acc`) over up to kDotTerms pairs, one pass,
 // one thread per element.  The pseudo-Mersenne primes sum the Karatsuba
 // products P1 = a0 b0, P2 = a1 b1, P3 = (a0 + a1)(b0 + b1) (each below 2^128:
-// a0 + a1, b0 + b1 < 2^64) in three 192-bit accumulators and reduce once per
-// element: re = P1 - P2, im = P3 - P1 - P2.  64 terms stay below 2^134, inside
-// red192's t < 2^8 bound, and red192 needs 2^64 mod p < 2^32, which holds for
-// these primes.  Other primes reduce every product.  Each element is read
-// completely before its output is written, so c may alias any operand of the
-// launch.
+// a0 + a1, b0 + b1 < 2^64) in three sums (ProductSum) and reduce each once per
+// element: re = P1 - P2, im = P3 - P1 - P2.  64 terms stay below 2^134, the
+// bound of a long ProductSum.  Other primes reduce every product.  Each element
+// is read completely before its output is written, so c may alias any operand of
+// the launch.
 struct DotArgs {
   const u2* a[kDotTerms];
   const u2* b[kDotTerms];

@@ -226,7 +226,6 @@ void prescale_factors(const Engine& e, std::vector<uint64_t>& pre0, std::vector<
   }
 }
 
-// f(i, arg) for i in [0, n) on the host's threads (shared with tdgt_tables.cu).
 void parallel_for_host(int n, void (*f)(int, void*), void* arg) {
   parallel_for(n, [&](int i) { f(i, arg); });
 }

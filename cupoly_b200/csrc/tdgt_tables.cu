@@ -10,9 +10,6 @@
 
 namespace cpoly {
 
-void prescale_factors(const Engine& e, std::vector<uint64_t>& pre0, std::vector<uint64_t>& pre1);
-void parallel_for_host(int n, void (*f)(int, void*), void* arg);
-
 namespace {
 
 int brev(int x, int bits) {
