@@ -17,6 +17,7 @@ struct FwdIO {
   ulonglong2* scatter[3];
   int src_polys;
   long long src_shift;
+  bool spread() const { return scatter[0] || src_polys; }
 };
 
 // Grid of a DGT launch.  When only one CTA fits per SM (N = 8192 in one CTA)
@@ -55,12 +56,13 @@ int run_cta(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglon
     return 1;
   }
   if (!inverse) {
-    static std::atomic<unsigned long long> done{0};
-    static std::atomic<int> resident{0};
-    if (int rc = ensure_smem(k_dgt_fwd<LOGNC, LOGR>, smem, done)) return rc;
-    const unsigned grid = persistent_grid(k_dgt_fwd<LOGNC, LOGR>, T, smem, resident, blocks);
-    k_dgt_fwd<LOGNC, LOGR><<<grid, T, smem, st>>>(data, fio.src, A, nres, rid_off, poly_stride, S, twist ? 1 : 0,
-                                                  (unsigned)blocks);
+    static std::atomic<unsigned long long> done[2];
+    static std::atomic<int> resident[2];
+    const int f = fio.spread() ? 1 : 0;
+    const auto kernel = f ? k_dgt_fwd<LOGNC, LOGR, 0, true> : k_dgt_fwd<LOGNC, LOGR, 0, false>;
+    if (int rc = ensure_smem(kernel, smem, done[f])) return rc;
+    const unsigned grid = persistent_grid(kernel, T, smem, resident[f], blocks);
+    kernel<<<grid, T, smem, st>>>(data, fio.src, A, nres, rid_off, poly_stride, S, twist ? 1 : 0, (unsigned)blocks);
   } else {
     static std::atomic<unsigned long long> done{0};
     static std::atomic<int> resident{0};
@@ -106,8 +108,8 @@ int run_cluster(const Engine& e, const DgtPlan&, const DgtTableLayout& L, ulongl
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  static std::atomic<unsigned long long> done_f{0}, done_i{0};
-  static std::atomic<int> ok_f{0}, ok_i{0};  // 0 unknown, 1 schedulable, -1 not
+  static std::atomic<unsigned long long> done_f[2], done_i{0};
+  static std::atomic<int> ok_f[2], ok_i{0};  // 0 unknown, 1 schedulable, -1 not
   auto schedulable = [&](auto kernel, std::atomic<int>& ok) {
     int v = ok.load();
     if (v == 0) {
@@ -121,10 +123,11 @@ int run_cluster(const Engine& e, const DgtPlan&, const DgtTableLayout& L, ulongl
   };
   cudaError_t err;
   if (!inverse) {
-    if (int rc = ensure_smem(k_dgt_fwd<LOGNC, LOGR, CL>, smem, done_f)) return rc;
-    if (!schedulable(k_dgt_fwd<LOGNC, LOGR, CL>, ok_f)) return kNoCluster;
-    err = cudaLaunchKernelEx(&cfg, k_dgt_fwd<LOGNC, LOGR, CL>, data, fio.src, A, nres, rid_off, poly_stride, CL, 1,
-                             (unsigned)blocks);
+    const int f = fio.spread() ? 1 : 0;
+    const auto kernel = f ? k_dgt_fwd<LOGNC, LOGR, CL, true> : k_dgt_fwd<LOGNC, LOGR, CL, false>;
+    if (int rc = ensure_smem(kernel, smem, done_f[f])) return rc;
+    if (!schedulable(kernel, ok_f[f])) return kNoCluster;
+    err = cudaLaunchKernelEx(&cfg, kernel, data, fio.src, A, nres, rid_off, poly_stride, CL, 1, (unsigned)blocks);
   } else {
     if (int rc = ensure_smem(k_dgt_inv<LOGNC, LOGR, CL>, smem, done_i)) return rc;
     if (!schedulable(k_dgt_inv<LOGNC, LOGR, CL>, ok_i)) return kNoCluster;
@@ -182,10 +185,9 @@ int launch_split(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulo
   }
   const int S = P.S, lc = P.logNc, lr = P.logR;
   if (!inverse) {
-    if (S == 1)
-      k_dgt_split<1, false><<<(unsigned)blocks, 256, 0, st>>>(data, fio.src, A, nres, rid_off, poly_stride, lc, lr);
-    else
-      k_dgt_split<2, false><<<(unsigned)blocks, 256, 0, st>>>(data, fio.src, A, nres, rid_off, poly_stride, lc, lr);
+    const auto kernel = fio.spread() ? (S == 1 ? k_dgt_split<1, false, true> : k_dgt_split<2, false, true>)
+                                     : (S == 1 ? k_dgt_split<1, false> : k_dgt_split<2, false>);
+    kernel<<<(unsigned)blocks, 256, 0, st>>>(data, fio.src, A, nres, rid_off, poly_stride, lc, lr);
   } else {
     if (S == 1)
       k_dgt_split<1, true><<<(unsigned)blocks, 256, 0, st>>>(data, nullptr, A, nres, rid_off, poly_stride, lc, lr);
@@ -310,7 +312,7 @@ int launch_dgt_ex(const Engine& e, void* dst_v, const void* fsrc_v, const InvSrc
 
 // Forward transforms of npolys polynomials at a into dst and npolys at b behind them, in one launch
 // where both launches would run the same CUDA-core plan: a small call's time is its launches'
-// (nphi 4096, 2 residues, one product: 33.6 us with two, 24.6 us with one).
+// (nphi 4096, 2 residues, one product: 32.8 us with two, 22.5 us with one; on another card 33.8 and 24.6).
 int launch_dgt_pair(const Engine& e, void* dst_v, const void* a_v, const void* b_v, int base, int npolys,
                     cudaStream_t st) {
   const int nres = e.n_residues(base);

@@ -174,6 +174,10 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   }
 }
 
+// Forward transforms that scatter their results or have two sources (DgtArgs) are the SPREAD form of the
+// kernels: in the plain form the selects and the arguments behind them cost a small launch
+// 0.25 to 0.5 us (one residue at nphi 4096 7.1 -> 7.6 us, 5 at nphi 8192 8.7 -> 8.9).
+
 // Where polynomial `poly` of a forward transform is written (by selects, as inv_src_ptr).
 __device__ __forceinline__ ulonglong2* fwd_dst(const DgtArgs& A, ulonglong2* data, int poly, long long poly_stride) {
   if (!A.scatter[0]) return data + poly * poly_stride;
@@ -411,7 +415,7 @@ constexpr bool dgt_prefetches() {
 // CL > 0: the split stage of 2^CL chunks runs inside the kernel's thread-block
 // cluster (launched with cluster dimension 2^CL, one CTA per unit, S = CL); the
 // input is read untwisted and the twist applied here (cluster_split_fwd).
-template <int LOGNC, int LOGR, int CL = 0>
+template <int LOGNC, int LOGR, int CL = 0, bool SPREAD = false>
 __global__ void __launch_bounds__((1 << LOGNC) >> LOGR, (dgt_min_blocks<LOGNC, LOGR>()))
     k_dgt_fwd(ulonglong2* __restrict__ data, const ulonglong2* __restrict__ src_base, DgtArgs A, int nres,
               int rid_off, long long poly_stride, int S, int twist, unsigned nunits) {
@@ -433,7 +437,7 @@ __global__ void __launch_bounds__((1 << LOGNC) >> LOGR, (dgt_min_blocks<LOGNC, L
   for (unsigned ub = blockIdx.x; ub < nunits; ub += gridDim.x) {
   if (dgt_prefetches<LOGNC, LOGR, CL>() && tid == 0 && ub + gridDim.x < nunits) {
     const unsigned un = ub + gridDim.x;
-    prefetch_l2(in_base + unit_off(un) + src_shift(A, (int)(un >> S) / nres), NC * 16u);
+    prefetch_l2(in_base + unit_off(un) + (SPREAD ? src_shift(A, (int)(un >> S) / nres) : 0), NC * 16u);
   }
   const int pr = (int)(ub >> S);
   const int r = pr % nres;
@@ -441,9 +445,13 @@ __global__ void __launch_bounds__((1 << LOGNC) >> LOGR, (dgt_min_blocks<LOGNC, L
   const uint64_t p = A.mc[rid].p;
   const ulonglong2* tab = A.tab + (size_t)rid * A.stride;
   const size_t off = unit_off(ub);
-  const int poly = pr / nres;
-  ulonglong2* x = fwd_dst(A, data, poly, poly_stride) + (off - (size_t)poly * poly_stride);
-  const ulonglong2* xs = src_base ? src_base + off + src_shift(A, poly) : x;  // in place: the output's own place
+  ulonglong2* x = data + off;
+  const ulonglong2* xs = in_base + off;
+  if constexpr (SPREAD) {
+    const int poly = pr / nres;
+    x = fwd_dst(A, data, poly, poly_stride) + (off - (size_t)poly * poly_stride);
+    xs = src_base ? src_base + off + src_shift(A, poly) : x;  // in place: the output's own place
+  }
   for (int j = tid; j < R; j += T) srad[j] = tab[A.L.off_rad + j];
   stage_twiddles<LOGNC, LOGR>(stw, tab, A.L.off_fwd);
   __syncthreads();
@@ -672,7 +680,7 @@ __global__ void __launch_bounds__((1 << LOGNC) >> LOGR, (dgt_min_blocks<LOGNC, L
 
 // Element-wise top stage for N = 2^S * Nc (forward: twist + radix-2^S DIF
 // over the top S bits + twiddle; inverse: twiddle + radix-2^S DIT + untwist).
-template <int S, bool INV>
+template <int S, bool INV, bool SPREAD = false>
 __global__ void __launch_bounds__(256)
     k_dgt_split(ulonglong2* __restrict__ data, const ulonglong2* __restrict__ src_base, DgtArgs A, int nres,
                 int rid_off, long long poly_stride, int logNc, int logR) {
@@ -685,8 +693,9 @@ __global__ void __launch_bounds__(256)
   const int rid = A.rid_list ? A.rid_list[pr] : rid_off + r;
   const uint64_t p = A.mc[rid].p;
   const ulonglong2* tab = A.tab + (size_t)rid * A.stride;
-  ulonglong2* x = (INV ? data + poly * poly_stride : fwd_dst(A, data, poly, poly_stride)) + ((size_t)r << (logNc + S));
-  const ulonglong2* xs = src_base ? src_base + poly * poly_stride + src_shift(A, poly) + ((size_t)r << (logNc + S)) : x;
+  ulonglong2* x = (SPREAD ? fwd_dst(A, data, poly, poly_stride) : data + poly * poly_stride) + ((size_t)r << (logNc + S));
+  const ulonglong2* xs = (src_base ? src_base : data) + poly * poly_stride + ((size_t)r << (logNc + S));
+  if (SPREAD) xs = src_base ? xs + src_shift(A, poly) : x;
   constexpr int K = 1 << S;
   uint64_t xr[K], xi[K];
   const int R = 1 << logR;
