@@ -11,13 +11,16 @@ namespace {
 
 // Input and output of a forward transform: `src` (nullptr: in place), and the places of
 // polynomials 0..2 (scatter[0] nullptr: all at the launch's data); src_polys, src_shift: a second
-// source array (see DgtArgs).
+// source array (see DgtSpreadArgs).
 struct FwdIO {
   const ulonglong2* src;
   ulonglong2* scatter[3];
   int src_polys;
   long long src_shift;
   bool spread() const { return scatter[0] || src_polys; }
+  DgtSpreadArgs args(const DgtArgs& A) const {
+    return DgtSpreadArgs{A, {scatter[0], scatter[1], scatter[2]}, src_polys, src_shift};
+  }
 };
 
 // Grid of a DGT launch.  When only one CTA fits per SM (N = 8192 in one CTA)
@@ -46,8 +49,7 @@ int run_cta(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglon
             cudaStream_t st, const int* rid_list) {
   constexpr int T = (1 << LOGNC) >> LOGR;
   constexpr int smem = dgt_smem_bytes<LOGNC, LOGR>();
-  DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list, {fio.scatter[0], fio.scatter[1], fio.scatter[2]},
-            fio.src_polys, fio.src_shift};
+  const DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list};
   const int S = P.S;
   const long long blocks = (long long)npolys * nres << S;
   if (blocks <= 0) return 0;
@@ -58,11 +60,15 @@ int run_cta(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglon
   if (!inverse) {
     static std::atomic<unsigned long long> done[2];
     static std::atomic<int> resident[2];
-    const int f = fio.spread() ? 1 : 0;
-    const auto kernel = f ? k_dgt_fwd<LOGNC, LOGR, 0, true> : k_dgt_fwd<LOGNC, LOGR, 0, false>;
-    if (int rc = ensure_smem(kernel, smem, done[f])) return rc;
-    const unsigned grid = persistent_grid(kernel, T, smem, resident[f], blocks);
-    kernel<<<grid, T, smem, st>>>(data, fio.src, A, nres, rid_off, poly_stride, S, twist ? 1 : 0, (unsigned)blocks);
+    auto launch = [&](auto kernel, const auto& args, int f) {
+      if (int rc = ensure_smem(kernel, smem, done[f])) return rc;
+      const unsigned grid = persistent_grid(kernel, T, smem, resident[f], blocks);
+      kernel<<<grid, T, smem, st>>>(data, fio.src, args, nres, rid_off, poly_stride, S, twist ? 1 : 0, (unsigned)blocks);
+      return 0;
+    };
+    const int rc = fio.spread() ? launch(k_dgt_fwd<LOGNC, LOGR, 0, true>, fio.args(A), 1)
+                                : launch(k_dgt_fwd<LOGNC, LOGR, 0, false>, A, 0);
+    if (rc) return rc;
   } else {
     static std::atomic<unsigned long long> done{0};
     static std::atomic<int> resident{0};
@@ -88,8 +94,7 @@ int run_cluster(const Engine& e, const DgtPlan&, const DgtTableLayout& L, ulongl
                 cudaStream_t st, const int* rid_list) {
   constexpr int T = (1 << LOGNC) >> LOGR;
   constexpr int smem = dgt_smem_bytes<LOGNC, LOGR>();
-  DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list, {fio.scatter[0], fio.scatter[1], fio.scatter[2]},
-            fio.src_polys, fio.src_shift};
+  const DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list};
   const long long blocks = (long long)npolys * nres << CL;
   if (blocks <= 0) return 0;
   if (blocks > 0x7fffffffLL) {
@@ -123,11 +128,15 @@ int run_cluster(const Engine& e, const DgtPlan&, const DgtTableLayout& L, ulongl
   };
   cudaError_t err;
   if (!inverse) {
-    const int f = fio.spread() ? 1 : 0;
-    const auto kernel = f ? k_dgt_fwd<LOGNC, LOGR, CL, true> : k_dgt_fwd<LOGNC, LOGR, CL, false>;
-    if (int rc = ensure_smem(kernel, smem, done_f[f])) return rc;
-    if (!schedulable(kernel, ok_f[f])) return kNoCluster;
-    err = cudaLaunchKernelEx(&cfg, kernel, data, fio.src, A, nres, rid_off, poly_stride, CL, 1, (unsigned)blocks);
+    auto launch = [&](auto kernel, const auto& args, int f) {
+      if (int rc = ensure_smem(kernel, smem, done_f[f])) return rc;
+      if (!schedulable(kernel, ok_f[f])) return kNoCluster;
+      err = cudaLaunchKernelEx(&cfg, kernel, data, fio.src, args, nres, rid_off, poly_stride, CL, 1, (unsigned)blocks);
+      return 0;
+    };
+    const int rc = fio.spread() ? launch(k_dgt_fwd<LOGNC, LOGR, CL, true>, fio.args(A), 1)
+                                : launch(k_dgt_fwd<LOGNC, LOGR, CL, false>, A, 0);
+    if (rc) return rc;
   } else {
     if (int rc = ensure_smem(k_dgt_inv<LOGNC, LOGR, CL>, smem, done_i)) return rc;
     if (!schedulable(k_dgt_inv<LOGNC, LOGR, CL>, ok_i)) return kNoCluster;
@@ -175,8 +184,7 @@ RunFn pick(int logNc, int logR) {
 int launch_split(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulonglong2* data, const FwdIO& fio,
                  int nres, int rid_off, int npolys, long long poly_stride, bool inverse, cudaStream_t st,
                  const int* rid_list = nullptr) {
-  DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list, {fio.scatter[0], fio.scatter[1], fio.scatter[2]},
-            fio.src_polys, fio.src_shift};
+  const DgtArgs A{e.d_tab, L.stride, L, e.d_mc, rid_list};
   const int Nc = 1 << P.logNc;
   const long long blocks = (long long)npolys * nres * (Nc / 256);
   if (blocks > 0x7fffffffLL) {
@@ -185,9 +193,13 @@ int launch_split(const Engine& e, const DgtPlan& P, const DgtTableLayout& L, ulo
   }
   const int S = P.S, lc = P.logNc, lr = P.logR;
   if (!inverse) {
-    const auto kernel = fio.spread() ? (S == 1 ? k_dgt_split<1, false, true> : k_dgt_split<2, false, true>)
-                                     : (S == 1 ? k_dgt_split<1, false> : k_dgt_split<2, false>);
-    kernel<<<(unsigned)blocks, 256, 0, st>>>(data, fio.src, A, nres, rid_off, poly_stride, lc, lr);
+    if (fio.spread()) {
+      const auto kernel = S == 1 ? k_dgt_split<1, false, true> : k_dgt_split<2, false, true>;
+      kernel<<<(unsigned)blocks, 256, 0, st>>>(data, fio.src, fio.args(A), nres, rid_off, poly_stride, lc, lr);
+    } else {
+      const auto kernel = S == 1 ? k_dgt_split<1, false> : k_dgt_split<2, false>;
+      kernel<<<(unsigned)blocks, 256, 0, st>>>(data, fio.src, A, nres, rid_off, poly_stride, lc, lr);
+    }
   } else {
     if (S == 1)
       k_dgt_split<1, true><<<(unsigned)blocks, 256, 0, st>>>(data, nullptr, A, nres, rid_off, poly_stride, lc, lr);

@@ -174,17 +174,20 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   }
 }
 
-// Forward transforms that scatter their results or have two sources (DgtArgs) are the SPREAD form of the
-// kernels: in the plain form the selects and the arguments behind them cost a small launch
-// 0.25 to 0.5 us (one residue at nphi 4096 7.1 -> 7.6 us, 5 at nphi 8192 8.7 -> 8.9).
+// Forward transforms that scatter their results or have two sources are the SPREAD form of the kernels
+// (DgtSpreadArgs): in the plain form the selects cost a small launch 0.25 to 0.5 us (one residue at nphi
+// 4096 7.1 -> 7.6 us, 5 at nphi 8192 8.7 -> 8.9), and the longer arguments alone changed the registers of the
+// plain kernels (split stage 54 -> 70).
+template <bool SPREAD>
+using FwdArgs = std::conditional_t<SPREAD, DgtSpreadArgs, DgtArgs>;
 
 // Where polynomial `poly` of a forward transform is written (by selects, as inv_src_ptr).
-__device__ __forceinline__ ulonglong2* fwd_dst(const DgtArgs& A, ulonglong2* data, int poly, long long poly_stride) {
+__device__ __forceinline__ ulonglong2* fwd_dst(const DgtSpreadArgs& A, ulonglong2* data, int poly, long long poly_stride) {
   if (!A.scatter[0]) return data + poly * poly_stride;
   return poly == 0 ? A.scatter[0] : poly == 1 ? A.scatter[1] : A.scatter[2];
 }
-// The second source's distance (DgtArgs::src_polys).
-__device__ __forceinline__ long long src_shift(const DgtArgs& A, int poly) {
+// The second source's distance (DgtSpreadArgs::src_polys).
+__device__ __forceinline__ long long src_shift(const DgtSpreadArgs& A, int poly) {
   return A.src_polys && poly >= A.src_polys ? A.src_shift : 0;
 }
 
@@ -417,7 +420,7 @@ constexpr bool dgt_prefetches() {
 // input is read untwisted and the twist applied here (cluster_split_fwd).
 template <int LOGNC, int LOGR, int CL = 0, bool SPREAD = false>
 __global__ void __launch_bounds__((1 << LOGNC) >> LOGR, (dgt_min_blocks<LOGNC, LOGR>()))
-    k_dgt_fwd(ulonglong2* __restrict__ data, const ulonglong2* __restrict__ src_base, DgtArgs A, int nres,
+    k_dgt_fwd(ulonglong2* __restrict__ data, const ulonglong2* __restrict__ src_base, FwdArgs<SPREAD> A, int nres,
               int rid_off, long long poly_stride, int S, int twist, unsigned nunits) {
   constexpr int NC = 1 << LOGNC, R = 1 << LOGR, T = NC >> LOGR;
   using C = PassCfg<LOGNC, LOGR>;
@@ -437,7 +440,9 @@ __global__ void __launch_bounds__((1 << LOGNC) >> LOGR, (dgt_min_blocks<LOGNC, L
   for (unsigned ub = blockIdx.x; ub < nunits; ub += gridDim.x) {
   if (dgt_prefetches<LOGNC, LOGR, CL>() && tid == 0 && ub + gridDim.x < nunits) {
     const unsigned un = ub + gridDim.x;
-    prefetch_l2(in_base + unit_off(un) + (SPREAD ? src_shift(A, (int)(un >> S) / nres) : 0), NC * 16u);
+    const ulonglong2* next = in_base + unit_off(un);
+    if constexpr (SPREAD) next += src_shift(A, (int)(un >> S) / nres);
+    prefetch_l2(next, NC * 16u);
   }
   const int pr = (int)(ub >> S);
   const int r = pr % nres;
@@ -682,7 +687,7 @@ __global__ void __launch_bounds__((1 << LOGNC) >> LOGR, (dgt_min_blocks<LOGNC, L
 // over the top S bits + twiddle; inverse: twiddle + radix-2^S DIT + untwist).
 template <int S, bool INV, bool SPREAD = false>
 __global__ void __launch_bounds__(256)
-    k_dgt_split(ulonglong2* __restrict__ data, const ulonglong2* __restrict__ src_base, DgtArgs A, int nres,
+    k_dgt_split(ulonglong2* __restrict__ data, const ulonglong2* __restrict__ src_base, FwdArgs<SPREAD> A, int nres,
                 int rid_off, long long poly_stride, int logNc, int logR) {
   const int Nc = 1 << logNc;
   const int chunks = Nc / 256;
@@ -693,9 +698,12 @@ __global__ void __launch_bounds__(256)
   const int rid = A.rid_list ? A.rid_list[pr] : rid_off + r;
   const uint64_t p = A.mc[rid].p;
   const ulonglong2* tab = A.tab + (size_t)rid * A.stride;
-  ulonglong2* x = (SPREAD ? fwd_dst(A, data, poly, poly_stride) : data + poly * poly_stride) + ((size_t)r << (logNc + S));
+  ulonglong2* x = data + poly * poly_stride + ((size_t)r << (logNc + S));
   const ulonglong2* xs = (src_base ? src_base : data) + poly * poly_stride + ((size_t)r << (logNc + S));
-  if (SPREAD) xs = src_base ? xs + src_shift(A, poly) : x;
+  if constexpr (SPREAD) {
+    x = fwd_dst(A, data, poly, poly_stride) + ((size_t)r << (logNc + S));
+    xs = src_base ? xs + src_shift(A, poly) : x;
+  }
   constexpr int K = 1 << S;
   uint64_t xr[K], xi[K];
   const int R = 1 << logR;

@@ -65,6 +65,9 @@ struct DgtArgs {
   DgtTableLayout L;
   const ModConst* mc;      // per engine residue
   const int* rid_list;     // work list: residue i of the data uses engine prime rid_list[i] (nullptr: base order)
+};
+// Forward transforms that scatter their results or have two sources.
+struct DgtSpreadArgs : DgtArgs {
   ulonglong2* scatter[3];  // forward output of polynomials 0..2 (scatter[0] nullptr: at `data`)
   // Out of place, polynomials from src_polys on are read src_shift elements further: a second
   // source array (0: there is none).
