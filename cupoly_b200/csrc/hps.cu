@@ -857,14 +857,17 @@ int launch_ss_n(ulonglong2* out, const ulonglong2* q, const SimpleArgs& a, cudaS
   return check_launch("simple_scaling");
 }
 
-// Whether `npolys` conversions from `ns` residues run on the tensor cores.  From 4 residues on
-// they are faster at every batch size (whole chain, nphi 8192, us: k 4, 2 pairs 74 -> 71, 256 pairs
-// 2097 -> 1921); with 1 or 2 the dot products are too short to be worth the operand's way through
-// shared memory (k 1, 256 pairs 703 against 766); with 3 they gain in large batches (8 pairs
-// 96.3 against 97.3, 64 pairs 466 -> 447).
-bool conv_on_tensor(const Engine& e, int ns, int npolys) {
+// Whether `npolys` conversions from `ns` residues to `ndst` run on the tensor cores.  From 5 residues
+// on, or 4 to more than 4, they are faster at every batch size (whole chain, nphi 8192, us: k 5, 1 pair 71.1 ->
+// 68.3; k 4, 1 pair 68.8 -> 67.4, 128 pairs 1015 -> 925); with 1 or 2 the dot products are too short to be
+// worth the operand's way through shared memory (k 1, 256 pairs 703 against 766).  Between, they gain
+// in large batches: 4 residues to 3 or 4 from 2^17 elements on (k 4, kl 4, 4 pairs 86.4 against 89.0, 8 pairs
+// 96.2 -> 94.3; k 3, 1 pair 64.5 against 65.5), 3 residues from 2^18 (8 pairs 96.3 against 97.3, 64
+// pairs 466 -> 447).
+bool conv_on_tensor(const Engine& e, int ns, int ndst, int npolys) {
   if (!e.d_cmat || e.N < 128) return false;
-  return ns >= 4 || (ns == 3 && (long long)npolys * e.N >= 1 << 18);
+  const long long elements = (long long)npolys * e.N;
+  return ns >= 5 || (ns == 4 && (ndst > 4 || elements >= 1 << 17)) || (ns == 3 && elements >= 1 << 18);
 }
 
 template <int NS, bool SCALE, class Args>
@@ -962,7 +965,7 @@ int hps_basis_ext_pre(const Engine& e, void* out, const void* in, bool q_to_b, i
   const int ns = q_to_b ? e.k : e.kl;
   auto* o = reinterpret_cast<ulonglong2*>(out);
   auto* i = reinterpret_cast<const ulonglong2*>(in);
-  if (conv_on_tensor(e, ns, npolys)) {
+  if (conv_on_tensor(e, ns, a.ndst, npolys)) {
 #define CALL(n) (launch_conv_tensor<n, false, ConvArgs>(e, q_to_b ? 0 : 2, o, i, nullptr, a, a.ndst, npolys, st))
     CP_SWITCH_NS(ns, CALL)
 #undef CALL
@@ -1045,7 +1048,7 @@ int hps_scale_to_q_pre(const Engine& e, void* out_q, const void* in_q, const voi
   auto* q = reinterpret_cast<const ulonglong2*>(in_q);
   auto* b = reinterpret_cast<const ulonglong2*>(in_b);
   int rc;
-  if (conv_on_tensor(e, e.k, npolys)) {
+  if (conv_on_tensor(e, e.k, e.kl, npolys)) {
 #define CALL(n) (launch_conv_tensor<n, true, ScaleArgs>(e, 1, o, q, b, a, e.kl, npolys, st))
     rc = [&]() -> int { CP_SWITCH_NS(e.k, CALL) }();
 #undef CALL
