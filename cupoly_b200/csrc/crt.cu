@@ -66,6 +66,49 @@ __device__ __forceinline__ void crt_rows(ulonglong2* __restrict__ out, const uin
   }
 }
 
+// One thread per Gaussian element (coefficients j and j + N) of one residue, blockIdx.y its polynomial
+// and residue.  PM: every prime has 63 bits (BFV engines).
+template <bool PM>
+__global__ void __launch_bounds__(256) k_crt_direct(ulonglong2* __restrict__ out, const uint64_t* __restrict__ coefs,
+                                                    int nlimbs, int N, int nres, int rid_off,
+                                                    const ModConst* __restrict__ mc,
+                                                    const uint64_t* __restrict__ pow64,
+                                                    const uint64_t* __restrict__ pow64m) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= N) return;
+  const int y = blockIdx.y, rid = rid_off + y % nres;
+  const ModConst m = mc[rid];
+  const uint64_t* c0 = coefs + ((size_t)(y / nres) * 2 * N + j) * nlimbs;
+  const uint64_t* c1 = c0 + (size_t)N * nlimbs;
+  uint64_t a0 = 0, a1 = 0;
+  if (PM || m.pm) {
+    const uint64_t* w = pow64 + (size_t)rid * kMaxLimbs;
+    const uint32_t c = (uint32_t)((1ull << 63) - m.p);
+    ProductSum<true> x0, x1;
+    auto step = [&](int l) {
+      const uint64_t wl = __ldg(w + l);
+      x0.mac(c0[l], wl);
+      x1.mac(c1[l], wl);
+    };
+    if constexpr (PM) {
+#pragma unroll 4
+      for (int l = 0; l < nlimbs; ++l) step(l);
+    } else {
+      for (int l = 0; l < nlimbs; ++l) step(l);
+    }
+    a0 = canon(x0.fold(c), c, m.p);
+    a1 = canon(x1.fold(c), c, m.p);
+  } else {
+    const uint64_t* wm = pow64m + (size_t)rid * kMaxLimbs;
+    for (int l = 0; l < nlimbs; ++l) {
+      const uint64_t wl = __ldg(wm + l);
+      a0 = add_mod(a0, mont_mul(c0[l], wl, m.p, m.pneg), m.p);
+      a1 = add_mod(a1, mont_mul(c1[l], wl, m.p, m.pneg), m.p);
+    }
+  }
+  out[(size_t)y * N + j] = make_ulonglong2(a0, a1);
+}
+
 // Residues of T Gaussian elements (coefficients j and j + N) of polynomial blockIdx.y, four at a
 // time: groups blockIdx.z, blockIdx.z + gridDim.z, ... of the base.  The limbs are read once, in
 // order, into shared memory (rows of an odd number of words: no bank conflicts); one thread per
@@ -490,6 +533,28 @@ struct WireHeader {
 };
 static_assert(sizeof(WireHeader) == 64, "wire header is 64 bytes");
 
+// Whether cp_crt runs with a thread per element and residue (k_crt_direct) where the tensor cores do not
+// take it.  k_crt's blocks stage the limbs and then take the residues one after the other: with fewer blocks than
+// the SMs hold, with one residue (nothing is read twice) or with the long Montgomery chains of CKKS primes that
+// costs more than the limbs read again (us, k_crt / direct: nphi 8192, 5 residues and limbs, 1 polynomial 3.4 /
+// 2.4, 2 3.4 / 3.0, 4 3.6 / 3.5, 8 4.8 / 5.1; 1 residue of 6 limbs, 100 polynomials 12.9 / 9.9; CKKS, 6 residues of 7 limbs, 1
+// polynomial 6.7 / 3.1, 64 46 / 48; 24 of 25 limbs at nphi 32768, 4 polynomials 178 / 155).  Rows of a multiple of 8
+// words fall on few sets of L1 and favour k_crt (12 residues of 24 limbs, nphi 8192, 1 polynomial 7.1 / 10.8).
+bool crt_direct(const Engine& e, int nres, int nlimbs, int npolys) {
+  const long long blocks = (long long)npolys * nres * ((e.N + 255) / 256), sms = e.sms;
+  const bool strided = nlimbs % 8 == 0;
+  if (e.N < 128 && (nres > 2 || e.ckks_prec)) return e.ckks_prec || 4 * blocks <= (strided ? 9 : 16) * sms;
+  if (e.ckks_prec) {
+    if (!strided) return nres <= 2 || blocks <= 55 * sms;
+    if (nlimbs == 8) return blocks <= 4 * sms;
+    return nres >= 4 && 2 * blocks <= (nlimbs % 16 ? 5 : 2) * sms;
+  }
+  if (nres == 1) return nlimbs <= 7 || (nlimbs <= 12 && !strided && blocks <= 9 * sms);
+  if (blocks <= sms && (nlimbs <= 14 || (nlimbs % 16 && nlimbs <= (nres >= 4 ? 40 : nres == 3 ? 23 : 0)))) return true;
+  if (4 * blocks <= 11 * sms && nlimbs <= (nres >= 4 ? 7 : 6)) return true;
+  return blocks <= 2 * sms && nres >= 4 && nlimbs <= 12 && !strided;
+}
+
 uint32_t inv_small(int d) { return d < 2 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d); }  // see div_small
 
 const uint64_t* base_primes(const Engine& e, int base, uint64_t* tmp) {
@@ -611,8 +676,10 @@ int cp_crt(const cp_engine* h, void* out, const uint64_t* coefs, int nlimbs, int
     const long long tiles = (long long)npolys * (e.N / 128);
     const int smem = std::max(2 * 128 * kb + kb * ConvShape{nlimbs, nres}.cols(), 46 * 1024);
     // Below some 16 K tile x limb x residue steps the CUDA cores are faster (us, 5 limbs and residues:
-    // 512 tiles 6.8 there and 7.7 here, 4096 tiles 36 and 23; 12: 128 tiles 7.9 and 7.2, 512 tiles 20 and 11).
-    if (smem <= 200 * 1024 && tiles * nlimbs * nres >= 16384) {
+    // 512 tiles 6.8 there and 7.7 here, 4096 tiles 36 and 23; 12: 128 tiles 7.9 and 7.2, 512 tiles 20 and 11); with
+    // two residues below 32 K (7 limbs, 1600 tiles 6 % faster there, 2560 tiles as fast), with one always (6 limbs, 3200
+    // tiles 9.9 and 14.1, 8000 tiles 27 and 32).
+    if (smem <= 200 * 1024 && nres > 1 && tiles * nlimbs * nres >= (nres == 2 ? 32768 : 16384)) {
       static std::atomic<unsigned long long> done{0};
       if (int rc = ensure_smem(k_crt_tensor, 200 * 1024, done)) return rc;
       const IoTensor io{e.d_io, e.io_cols, e.N / 128, (int)tiles, inv_small(nlimbs), e.d_err};
@@ -621,6 +688,13 @@ int cp_crt(const cp_engine* h, void* out, const uint64_t* coefs, int nlimbs, int
                                                                nres, e.rid_offset(base), e.d_mc, io);
       return check_launch("cp_crt");
     }
+  }
+  if (crt_direct(e, nres, nlimbs, npolys)) {
+    const auto direct = e.ckks_prec ? k_crt_direct<false> : k_crt_direct<true>;
+    direct<<<dim3((e.N + 255) / 256, npolys * nres), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<ulonglong2*>(out), coefs, nlimbs, e.N, nres, e.rid_offset(base), e.d_mc, e.d_hps + e.ho.pow64,
+        e.d_hps + e.ho.pow64m);
+    return check_launch("cp_crt");
   }
   // elements per block: the limbs take at most 48 KB
   const int T = nlimbs <= 23 ? 128 : (nlimbs <= 47 ? 64 : 32);

@@ -1,6 +1,7 @@
-"""Tensor-core coefficient I/O over what its rule lets in: cp_crt over B and QB (a column offset into the
+"""Coefficient I/O over what its rules let in.  On the tensor cores: cp_crt over B and QB (a column offset into the
 matrix, up to six groups of columns), cp_icrt of B and of CKKS bases (a 63-bit prime beside shorter
-ones), and wide bases with more tiles than the grid has blocks.  Exact against Python integers."""
+ones), and wide bases with more tiles than the grid has blocks.  On the CUDA cores: cp_crt on both sides of the
+lines between a thread per element and residue and blocks that stage the limbs.  Exact against Python integers."""
 import numpy as np
 import pytest
 
@@ -74,3 +75,27 @@ def test_icrt_of_ckks_bases(gpu, prec, k, kl, nphi, npolys, base):
     ns, tiles = len(primes), npolys * (nphi // 256)
     assert 5 <= ns <= 16 and (ns >= 8 or tiles * ns * ns >= 32768)  # cp_icrt's tensor-core rule
     _check(e, base, primes, npolys, nphi, ns, sorted({0, npolys // 2, npolys - 1}))
+
+
+# (prec, k, nphi, polynomials, limbs): blocks of 256 elements x residues around 148, 296, 370 and 407, limb counts
+# around 7, 12, 14, 23 and 40 and multiples of 8 and 16, rings below one block, one and two residues, CKKS primes
+@pytest.mark.parametrize("prec,k,nphi,npolys,nlimbs", [
+    (0, 3, 4, 1, 3), (0, 5, 64, 118, 5), (0, 5, 64, 119, 5), (0, 5, 64, 66, 8), (0, 5, 64, 67, 8), (0, 1, 2048, 40, 7),
+    (0, 1, 2048, 40, 8), (0, 1, 8192, 84, 12), (0, 2, 2048, 50, 6), (0, 2, 2048, 52, 6), (0, 4, 1024, 18, 14),
+    (0, 4, 1024, 19, 14), (0, 4, 512, 37, 23), (0, 3, 512, 49, 23), (0, 4, 512, 37, 40), (0, 4, 512, 37, 16),
+    (0, 4, 2048, 18, 12), (0, 7, 1024, 29, 7), (0, 7, 1024, 30, 7), (0, 2, 8192, 40, 13),
+    (55, 2, 64, 3, 40), (55, 4, 512, 3, 4), (55, 4, 512, 3, 8), (55, 8, 512, 19, 16), (45, 6, 2048, 30, 40),
+    (48, 6, 1024, 40, 7), (52, 2, 1024, 40, 3)])
+def test_crt_on_the_cuda_cores(gpu, prec, k, nphi, npolys, nlimbs):
+    from cupoly_b200.engine import Engine
+    e = Engine.ckks(k, 1, nphi, prec) if prec else Engine(k, 1, nphi, 256)
+    w = _limbs(k * 7 + nlimbs, npolys, nphi, nlimbs, O.prod(e.Q)) if nphi >= 8 else splitmix64(
+        3, 5, npolys * nphi * nlimbs).reshape(npolys, nphi, nlimbs)
+    from cupoly_b200.engine import from_u64, limbs_to_ints, to_u64
+    x = e.empty(0, npolys)
+    e.crt(x, from_u64(w), 0)
+    got = to_u64(x).reshape(npolys, k, nphi // 2, 2)
+    for q in sorted({0, npolys // 2, npolys - 1}):
+        ints, res = limbs_to_ints(w[q]), unfold(got[q:q + 1])[0]
+        for r, p in enumerate(e.Q):
+            assert np.array_equal(res[r], np.array([v % p for v in ints], dtype=np.uint64)), (q, r)
