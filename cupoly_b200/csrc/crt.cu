@@ -33,6 +33,7 @@ namespace {
 constexpr int kCrtTensor = 32;    // most limbs of cp_crt on the tensor cores (256 bytes: column sums below 2^24)
 constexpr int kIcrtFirst = 5, kIcrtTensor = 16;  // primes of cp_icrt on the tensor cores (at most 256 columns of tensor memory)
 constexpr int kMaxIcrt = 24;  // largest base recombined by cp_icrt (|Q|, |B| <= 24)
+constexpr int kIcrtHeld = 15;  // primes whose digits and limbs k_icrt keeps in registers
 
 // i / d for i < 2^16, 2 <= d <= 64, with m = ceil(2^32 / d).
 __device__ __forceinline__ int div_small(int i, uint32_t m) { return (int)__umulhi((uint32_t)i, m); }
@@ -222,6 +223,52 @@ __global__ void __launch_bounds__(128) k_icrt(uint64_t* __restrict__ coefs, int 
   for (int i = tid & 63; i < nt * nlimbs; i += 64) {
     const int e = nlimbs == 1 ? i : div_small(i, inv_nlimbs), l = i - e * nlimbs;
     o[i] = l < NS ? s_x[(64 * half + e) * ROW + l] : 0;
+  }
+}
+
+// The same for a base of ns > kIcrtHeld primes, a coefficient's digits and limbs in one row of shared
+// memory: in registers they spill and the unrolled products no longer fit the instruction cache (us, 24
+// primes at nphi 8192, 1 polynomial: local memory 53, registers 70, so 50; 20 polynomials 166, 213, 152).  Digit i
+// lies at word i; when step i takes it, limbs 0 .. ns - 2 - i of X lie at words ns - 1 .. i + 1, and the limb
+// that the step adds takes its place.
+__global__ void __launch_bounds__(128) k_icrt_wide(uint64_t* __restrict__ coefs, int nlimbs,
+                                                   const ulonglong2* __restrict__ in, int N, int ns, int src_off,
+                                                   const ModConst* __restrict__ mc, const uint64_t* __restrict__ inv,
+                                                   const uint64_t* __restrict__ inv_s, uint32_t inv_nlimbs) {
+  constexpr int ROW = kMaxIcrt | 1;
+  __shared__ uint64_t s_x[128 * ROW];
+  const int tid = threadIdx.x, half = tid >> 6, j0 = blockIdx.x * 64, nt = N - j0 < 64 ? N - j0 : 64;
+  const int j = j0 + (tid & 63);
+  if ((tid & 63) < nt) {
+    uint64_t* x = s_x + tid * ROW;
+    const uint64_t* src = reinterpret_cast<const uint64_t*>(in + (size_t)blockIdx.y * ns * N + j) + half;
+    for (int i = 0; i < ns; ++i) {
+      const uint64_t si = mc[src_off + i].p;
+      uint64_t y = src[(size_t)i * 2 * N];
+      for (int l = 0; l < i; ++l) {
+        uint64_t dl = x[l];
+        if (dl >= si) dl = dl - si < si ? dl - si : dl % si;
+        const int c = i * (i - 1) / 2 + l;
+        y = shoup_mul(y + si - dl, __ldg(inv + c), __ldg(inv_s + c), si);
+      }
+      x[i] = y;
+    }
+    for (int i = ns - 2; i >= 0; --i) {
+      const uint64_t si = mc[src_off + i].p;
+      uint64_t carry = x[i];
+      for (int w = ns - 1; w > i; --w) {
+        const uint64_t v = x[w], lo = v * si, s = lo + carry;
+        carry = mulhi64(v, si) + (s < lo);
+        x[w] = s;
+      }
+      x[i] = carry;
+    }
+  }
+  __syncthreads();
+  uint64_t* o = coefs + ((size_t)blockIdx.y * 2 * N + j0 + (size_t)half * N) * nlimbs;
+  for (int i = tid & 63; i < nt * nlimbs; i += 64) {
+    const int e = div_small(i, inv_nlimbs), l = i - e * nlimbs;
+    o[i] = l < ns ? s_x[(64 * half + e) * ROW + ns - 1 - l] : 0;
   }
 }
 
@@ -745,8 +792,12 @@ int cp_icrt(const cp_engine* h, uint64_t* coefs, int nlimbs, const void* in, int
   }
   const uint64_t* inv = e.d_hps + (base == CP_QBASE ? e.ho.qb_inv : e.ho.bq_inv);
   const uint64_t* inv_s = e.d_hps + (base == CP_QBASE ? e.ho.qb_inv_s : e.ho.bq_inv_s);
-  icrt_kernel(ns, std::make_integer_sequence<int, kMaxIcrt>())<<<dim3((e.N + 63) / 64, npolys), 128, 0, st>>>(
-      coefs, nlimbs, src, e.N, e.rid_offset(base), e.d_mc, inv, inv_s, inv_small(nlimbs));
+  if (ns > kIcrtHeld)
+    k_icrt_wide<<<dim3((e.N + 63) / 64, npolys), 128, 0, st>>>(coefs, nlimbs, src, e.N, ns, e.rid_offset(base), e.d_mc,
+                                                               inv, inv_s, inv_small(nlimbs));
+  else
+    icrt_kernel(ns, std::make_integer_sequence<int, kIcrtHeld>())<<<dim3((e.N + 63) / 64, npolys), 128, 0, st>>>(
+        coefs, nlimbs, src, e.N, e.rid_offset(base), e.d_mc, inv, inv_s, inv_small(nlimbs));
   return check_launch("cp_icrt");
 }
 

@@ -99,3 +99,15 @@ def test_crt_on_the_cuda_cores(gpu, prec, k, nphi, npolys, nlimbs):
         ints, res = limbs_to_ints(w[q]), unfold(got[q:q + 1])[0]
         for r, p in enumerate(e.Q):
             assert np.array_equal(res[r], np.array([v % p for v in ints], dtype=np.uint64)), (q, r)
+
+
+# more primes than are kept in registers (15), where the tensor cores (16 at most, N >= 128) do not take them: rings
+# below a block's 64 elements, most limbs, CKKS digits that need a division
+@pytest.mark.parametrize("prec,k,kl,nphi,npolys,nlimbs,base", [
+    (0, 16, 1, 16, 3, 16, 0), (0, 16, 1, 128, 5, 19, 0), (0, 17, 1, 64, 2, 17, 0), (0, 19, 1, 512, 30, 25, 0),
+    (0, 24, 24, 1024, 40, 24, 1), (0, 24, 24, 256, 3, 64, 0), (45, 17, 1, 256, 3, 17, 0), (55, 24, 1, 512, 20, 25, 0),
+    (52, 20, 18, 64, 7, 20, 1)])
+def test_icrt_of_wide_bases(gpu, prec, k, kl, nphi, npolys, nlimbs, base):
+    from cupoly_b200.engine import Engine
+    e = Engine.ckks(k, kl, nphi, prec) if prec else Engine(k, kl, nphi, 256)
+    _check(e, base, e.base_primes(base), npolys, nphi, nlimbs, sorted({0, npolys // 2, npolys - 1}))
