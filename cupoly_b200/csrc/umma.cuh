@@ -28,8 +28,8 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 }
 
 constexpr uint32_t kWaitPolls = 1u << 20;         // each poll suspends for the hardware's own time limit
-constexpr uint64_t kWaitNs = 2000000000ull;       // and no wait lasts longer than 2 s,
-constexpr uint32_t kWaitLeast = 1u << 10;         // except for these polls: the clock runs on while the context is
+constexpr uint64_t kWaitNs = 2000000000ull;       // and no wait lasts much longer than 2 s, by a clock that is
+constexpr uint32_t kWaitLook = 1u << 8;           // looked at after so many polls: it runs on while the context is
                                                   // switched out, the copies and products waited for do not
 
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
@@ -43,24 +43,26 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 }
 // Waits until the phase of the given parity has completed; see the file comment for the bound.
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatile int* fail) {
-  if (mbar_try(bar, parity) || *fail) return;
+  if (mbar_try(bar, parity)) return;
   uint64_t t0 = 0;
   for (uint32_t i = 0; i < kWaitPolls; ++i) {
     if (mbar_try(bar, parity)) return;
-    if ((i & 15u) == 15u) {
+    if (i % kWaitLook == kWaitLook - 1) {
       uint64_t t;
       asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
       if (t0 == 0) t0 = t;
-      if (*fail || (i > kWaitLeast && t - t0 > kWaitNs)) break;
+      if (*fail || t - t0 > kWaitNs) break;
     }
   }
   *fail = 1;
 }
 // At a block's end, after a barrier of its threads and before its memory passes on: copies and
 // products may still be in flight if a wait ran out, and get 0.1 s to land.
+static __device__ __noinline__ void settle_slow() {
+  for (int i = 0; i < 100; ++i) __nanosleep(1000000);
+}
 __device__ __forceinline__ void settle(const volatile int* fail) {
-  if (*fail)
-    for (int i = 0; i < 100; ++i) __nanosleep(1000000);
+  if (*fail) settle_slow();
 }
 
 // Tensor memory: `ncols` (a power of two >= 32) 32-bit columns of 128 lanes, by one whole warp.
