@@ -42,7 +42,7 @@ SIGNATURES = {
     "cp_engine_set_plan": (_i, [_vp, _i, _i]),
     "cp_engine_set_tensor": (_i, [_vp, _i]),
     "cp_engine_get_tensor": (_i, [_vp]),
-    "cp_engine_dgt_launches": (_i, [_vp, C.c_longlong, _i, C.POINTER(_i)]),
+    "cp_engine_dgt_launches": (_i, [_vp, C.c_longlong, _i, C.POINTER(_i), C.POINTER(_i)]),
     "cp_engine_get_plan": (_i, [_vp, C.POINTER(_i), C.POINTER(_i), C.POINTER(_i)]),
     "cp_engine_check_async": (_i, [_vp, _vp, _vp]),
     "cp_engine_set_narrow_plan": (_i, [_vp, _i, _i, C.c_longlong]),

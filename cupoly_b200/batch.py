@@ -193,11 +193,11 @@ class MixedPolymul:
 
     def launches_per_run(self) -> int:
         """Launches of one run: per size group two forward transforms and an inverse (each counted as one,
-        whatever kernels its plan takes), and the products where the group runs on the tensor
-        cores."""
+        whatever kernels its plan takes), and the products where they are a kernel of their
+        own."""
         if self.mode == "tiles":
             return 1
-        return sum(3 + int(g["engine"].dgt_launches(g["rows"], work_list=True)[1]) for g in self.groups.values())
+        return sum(3 + int(g["engine"].products_apart(g["rows"], work_list=True)) for g in self.groups.values())
 
     def algorithmic_bytes(self) -> int:
         """24 nphi k bytes per product: read a, b and write c (16 B per Gaussian element)."""

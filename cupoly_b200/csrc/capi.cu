@@ -304,9 +304,10 @@ int cp_engine_set_split_mode(cp_engine* h, int mode) {
   return CP_OK;
 }
 
-int cp_engine_dgt_launches(const cp_engine* h, long long units, int work_list, int* on_tensor) {
+int cp_engine_dgt_launches(const cp_engine* h, long long units, int work_list, int* on_tensor, int* products_apart) {
   if (!h || units < 0) return -1;
-  if (on_tensor) *on_tensor = units > 0 && dgt_on_tensor(h->e, units, work_list != 0) ? 1 : 0;
+  if (on_tensor) *on_tensor = units > 0 && dgt_on_tensor(h->e, units, false, work_list != 0) ? 1 : 0;
+  if (products_apart) *products_apart = units > 0 && dgt_on_tensor(h->e, units, true, work_list != 0) ? 1 : 0;
   return dgt_launches(h->e, units, work_list != 0);
 }
 
@@ -449,7 +450,7 @@ int cp_polymul(const cp_engine* h, void* c, const void* a, const void* b, int ba
   InvSrc is{};
   is.p[0] = wa;
   is.npairs = 1;
-  if (dgt_on_tensor(e, (long long)npolys * e.n_residues(base))) {  // see tensor_inverse
+  if (dgt_on_tensor(e, (long long)npolys * e.n_residues(base), true)) {  // see tensor_inverse
     if (int rc = pw_mul(e, wa, wa, wb, base, st, npolys, true)) return rc;
   } else {
     is.p[1] = wb;
@@ -469,7 +470,7 @@ int cp_polymul_list(const cp_engine* h, void* c, const void* a, const void* b, v
   InvSrc is{};
   is.p[0] = reinterpret_cast<const ulonglong2*>(wa);
   is.npairs = 1;
-  if (dgt_on_tensor(e, nlist, true)) {  // see tensor_inverse
+  if (dgt_on_tensor(e, nlist, true, true)) {  // see tensor_inverse
     if (int rc = pw_mul_list(e, wa, wa, wb, rid_list, nlist, st, true)) return rc;
   } else {
     is.p[1] = reinterpret_cast<const ulonglong2*>(wb);
@@ -696,7 +697,7 @@ static int tensor_inverse(const Engine& e, ulonglong2* out, const ulonglong2* co
   const int nres = e.n_residues(base);
   InvSrc is{};
   is.untwist = untwist;
-  if (dgt_on_tensor(e, 3LL * npairs * nres)) {
+  if (dgt_on_tensor(e, 3LL * npairs * nres, true)) {
     const size_t one = (size_t)npairs * nres * e.N;
     CP_TRY(pw_dr2(e, out, out + one, out + 2 * one, p[0], p[1], p[2], p[3], base, st, npairs, true));
     is.p[0] = out;

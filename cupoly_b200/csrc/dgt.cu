@@ -230,8 +230,9 @@ namespace {
 // then the split stage.  With the cluster form the split stage runs inside the kernel.
 int run_transform(const Engine& e, ulonglong2* data, const FwdIO& fio, const InvSrc& isrc, int nres,
                   int rid_off, int npolys, long long poly_stride, bool inverse, cudaStream_t st, const int* rid_list) {
-  // the tensor-core kernel has one source and one output
-  if (!fio.scatter[0] && !fio.src_polys && dgt_on_tensor(e, (long long)npolys * nres, rid_list != nullptr)) {
+  // the tensor-core kernel has one source and one output, and forms no products
+  const bool products = inverse && (isrc.mode == 1 || isrc.mode == 3);
+  if (!fio.spread() && !products && dgt_on_tensor(e, (long long)npolys * nres, inverse, rid_list != nullptr)) {
     if (inverse && isrc.untwist > 2) {
       set_error("dgt: unknown untwist table");
       return 1;
@@ -285,15 +286,15 @@ int run_transform(const Engine& e, ulonglong2* data, const FwdIO& fio, const Inv
 
 }  // namespace
 
-bool dgt_on_tensor(const Engine& e, long long units, bool list) {
+bool dgt_on_tensor(const Engine& e, long long units, bool inverse, bool list) {
   if (!e.d_ttab || (list && e.tlayout.S > 0)) return false;
   if (e.tensor == 1 && (units <= e.narrow_first || (e.cluster_first && e.plan.S > 0))) return false;
-  return units > e.tensor_above;
+  return units > (list ? e.tensor_above_list[inverse ? 1 : 0] : e.tensor_above);
 }
 
 int dgt_launches(const Engine& e, long long units, bool list) {
   if (units <= 0) return 0;
-  if (dgt_on_tensor(e, units, list))
+  if (dgt_on_tensor(e, units, false, list))
     return list ? (int)((units + kTdgtListMax - 1) / kTdgtListMax) : (e.tlayout.S > 0 ? 2 : 1);
   const DgtPlan& P = select_plan(e, units).P;
   return P.S == 0 || (P.cluster && pick_cluster(P.logNc, P.logR, P.S)) ? 1 : 2;
@@ -337,7 +338,7 @@ int launch_dgt_pair(const Engine& e, void* dst_v, const void* a_v, const void* b
   const ulonglong2 *a = reinterpret_cast<const ulonglong2*>(a_v), *b = reinterpret_cast<const ulonglong2*>(b_v);
   const bool same_plan = &select_plan(e, units).P == &select_plan(e, 2 * units).P;
   // (large calls run on the tensor cores; a grid for both must not be refused where one was accepted)
-  if (dgt_on_tensor(e, 2 * units) || !same_plan || 2 * units * (e.N / 256 + 1) > 0x7fffffffLL) {
+  if (dgt_on_tensor(e, 2 * units, false) || !same_plan || 2 * units * (e.N / 256 + 1) > 0x7fffffffLL) {
     if (int rc = launch_dgt_ex(e, dst, a, nullptr, base, npolys, 0, false, st)) return rc;
     return launch_dgt_ex(e, dst + npolys * stride, b, nullptr, base, npolys, 0, false, st);
   }
@@ -356,7 +357,7 @@ int launch_dgt_scatter3(const Engine& e, void* const dst[3], const void* src_v, 
   }
   const ulonglong2* src = reinterpret_cast<const ulonglong2*>(src_v);
   const long long stride = (long long)nres * e.N;
-  if (dgt_on_tensor(e, nres)) {
+  if (dgt_on_tensor(e, nres, false)) {
     for (int v = 0; v < 3; ++v)
       if (int rc = launch_dgt_ex(e, dst[v], src + v * stride, nullptr, base, 1, 0, false, st)) return rc;
     return 0;

@@ -148,6 +148,7 @@ struct Engine {
   int tensor = 1;                  // transforms on the tensor cores: 0 never, 1 in launches of more than
                                    // tensor_above residue transforms, 2 always (cp_engine_set_tensor)
   int tensor_above = 0;
+  int tensor_above_list[2] = {0, 0};  // the same for work lists: forward, inverse
   // Plan settings made after the last cp_engine_set_tensor go before mode 1: launches of at most
   // narrow_first units keep the small-launch plan, cluster_first keeps the cluster form of the split stage.
   long long narrow_first = 0;
@@ -244,7 +245,7 @@ void parallel_for_host(int n, void (*f)(int, void*), void* arg);  // f(i, arg) f
 int build_io_tables(Engine& e);      // crt.cu
 int build_tensor_tables(Engine& e);  // tdgt_tables.cu; after the plans are placed
 bool tensor_possible(const Engine& e);  // whether those tables can be built beside the present plan
-void place_tensor_line(Engine& e);      // tensor_above of the present mode
+void place_tensor_line(Engine& e);      // tensor_above and tensor_above_list of the present mode
 void free_tables(Engine& e);
 
 }  // namespace cpoly

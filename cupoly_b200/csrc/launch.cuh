@@ -71,8 +71,8 @@ int launch_dgt_pair(const Engine& e, void* dst, const void* a, const void* b, in
 int launch_dgt_ex(const Engine& e, void* dst, const void* fsrc, const InvSrc* isrc, int base, int npolys,
                   long long poly_stride, bool inverse, cudaStream_t st);
 // Whether a launch of `units` residue transforms runs on the tensor cores.
-bool dgt_on_tensor(const Engine& e, long long units, bool list = false);
-// Kernels of a launch of `units` residue transforms.
+bool dgt_on_tensor(const Engine& e, long long units, bool inverse, bool list = false);
+// Kernels of a forward launch of `units` residue transforms.
 int dgt_launches(const Engine& e, long long units, bool list);
 // Forward transforms of three polynomials back to back in `src` into dst[0..2].
 int launch_dgt_scatter3(const Engine& e, void* const dst[3], const void* src, int base, cudaStream_t st);

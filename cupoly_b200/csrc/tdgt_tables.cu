@@ -143,7 +143,15 @@ void place_tensor_line(Engine& e) {
   // nphi 2048: 288 residues 19 / 24, 384 25 / 24; 4096: 64 18 / 23, 96 22 / 23, 148 24 / 23;
   // 8192: 32 19 / 24, 64 24 / 24; 16384: 32 28 / 44, 64 43 / 44; 32768: 1 36 / 31.
   static const int above[5] = {320, 96, 64, 64, 0};
-  e.tensor_above = e.tensor == 2 ? 0 : above[e.logN < 10 ? 0 : (e.logN < 14 ? e.logN - 10 : 4)];
+  // Rows of a work list fill a unit with residues of one prime only, load apart from each other at N = 1024, and are
+  // ordered first.  Forward / inverse of the list, us, CUDA cores; tensor cores: nphi 2048: 1000 rows 24 / 25.4; 27 /
+  // 25.1, 1600 37 / 39; 38 / 34, 2400 53 / 57; 57 / 50, 2800 60.5 / 63.5; 59 / 52; 4096: 140 rows 12.2 / 12.6; 13.9 /
+  // 13.5, 150 14.9 / 15.3; 14.0 / 13.6; 8192: 65 rows 12.6 / 13.0; 14.1 / 14.1, 75 16.0 / 16.4; 14.2 / 14.1; 16384:
+  // 65 21 / 22; 24 / 23, 75 27 / 28; 24 / 24.
+  static const int list_above[4][2] = {{2600, 1150}, {148, 148}, {74, 74}, {74, 74}};
+  const int at = e.logN < 10 ? 0 : (e.logN < 14 ? e.logN - 10 : 4);
+  e.tensor_above = e.tensor == 2 ? 0 : above[at];
+  for (int v = 0; v < 2; ++v) e.tensor_above_list[v] = e.tensor == 2 || at == 4 ? 0 : list_above[at][v];
 }
 
 // Places and fills the tensor-core tables when the engine can use them.

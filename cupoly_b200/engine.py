@@ -159,19 +159,25 @@ class Engine:
         return _lib.lib().cp_engine_get_tensor(self._h) == 1
 
     def dgt_launches(self, units: int, work_list: bool = False) -> Tuple[int, bool]:
-        """Kernels of one transform launch of `units` residue transforms, and whether they are the
-        tensor-core ones (where the products of a fused call are a kernel of their own)."""
+        """Kernels of one forward launch of `units` residue transforms, and whether they are the
+        tensor-core ones."""
         t = C.c_int()
-        n = _lib.lib().cp_engine_dgt_launches(self._h, int(units), 1 if work_list else 0, C.byref(t))
+        n = _lib.lib().cp_engine_dgt_launches(self._h, int(units), 1 if work_list else 0, C.byref(t), None)
         return n, t.value == 1
+
+    def products_apart(self, units: int, work_list: bool = False) -> bool:
+        """Whether the products of a fused call of `units` residues are a kernel of their own."""
+        p = C.c_int()
+        _lib.lib().cp_engine_dgt_launches(self._h, int(units), 1 if work_list else 0, None, C.byref(p))
+        return p.value == 1
 
     def bfv_mul_batch_launches(self, npairs: int) -> int:
         """Kernels of one bfv_mul_batch call: three base conversions, the transforms of 4 npairs inputs over
         Q and over B and of 3 npairs outputs over Q, over B and over Q again, and the products over a
-        base whose inverse runs on the tensor cores."""
+        base where they are a kernel of their own."""
         q, b = npairs * self.k, npairs * self.kl
         n = 3 + sum(self.dgt_launches(u)[0] for u in (4 * q, 4 * b, 3 * q, 3 * b, 3 * q))
-        return n + sum(int(self.dgt_launches(u)[1]) for u in (3 * q, 3 * b))
+        return n + int(self.products_apart(3 * q)) + int(self.products_apart(3 * b))
 
     def set_split_mode(self, mode: int):
         """0: split stage as its own kernel (HBM pass); 1: inside a thread-block cluster (DSMEM)."""

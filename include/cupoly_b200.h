@@ -105,10 +105,11 @@ int cp_engine_set_plan(cp_engine* e, int log_radix, int log_cta);
 int cp_engine_set_tensor(cp_engine* e, int mode);
 /* 1: the engine holds tensor-core tables; 0: it does not; -1: NULL engine. */
 int cp_engine_get_tensor(const cp_engine* e);
-/* Kernels that one transform launch of `units` residue transforms (polynomials x residues; work_list:
+/* Kernels that one forward launch of `units` residue transforms (polynomials x residues; work_list:
  * rows of a list) takes with the present settings; -1: NULL engine or units < 0.  *on_tensor (may be NULL): 1 when
- * they are the tensor-core ones, where the products of a fused call are a kernel of their own. */
-int cp_engine_dgt_launches(const cp_engine* e, long long units, int work_list, int* on_tensor);
+ * they are the tensor-core ones.  *products_apart (may be NULL): 1 when the products of a fused call (cp_polymul*,
+ * cp_bfv_mul*) are a kernel of their own before its inverse. */
+int cp_engine_dgt_launches(const cp_engine* e, long long units, int work_list, int* on_tensor, int* products_apart);
 int cp_engine_get_plan(const cp_engine* e, int* log_radix, int* log_cta, int* split_bits);
 /* Second DGT plan for small launches (no counterpart in cuPoly): a transform launch of at
  * most max_units residue transforms (polynomials x residues) uses (log_radix, log_cta)
