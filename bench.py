@@ -727,7 +727,7 @@ def run_ours(args, D: Dist):
     mixed_ms = mixed_forms[best]
     mixed = {"config": "1024 products, nphi uniform in {2048, 4096, 8192, 16384}, k uniform in 1..8 (seeded), "
                        "2 batches in flight; fastest of three forms: %s" % best,
-             "form": {"sequence": "one CUDA graph, per size group a fused cp_polymul_list (3 launches; 4 on the tensor cores)",
+             "form": {"sequence": "one CUDA graph, per size group a fused cp_polymul_list (3 launches, 4 with the products apart)",
                       "branches": "the same graph with one parallel branch per size group",
                       "tiles": "one persistent launch (cp_polymul_tiles) over a work list of tiles"}[best],
              "launches_per_batch": mixed_launches[best],

@@ -6,7 +6,8 @@ Instances are grouped by ring size; inside a group every residue of every
 instance is one entry of a work list (data pointer implied by its position,
 prime index = its residue number), and one fused `cp_polymul_list` serves the
 whole group whatever the mix of widths: an out-of-place forward DGT per
-operand and an inverse DGT that forms the products while loading.  All
+operand and an inverse DGT that forms the products while loading (a product
+kernel before it on the tensor cores).  All
 groups' launches are captured once in a CUDA graph and replayed (in sequence,
 or as one parallel branch per size group).  mode="tiles" runs the whole batch
 as ONE persistent launch instead (cp_polymul_tiles): one CTA per SM walks a

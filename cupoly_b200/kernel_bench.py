@@ -25,7 +25,7 @@ Workloads (names for --only):
                      polynomials, nphi 8192, k 5; bytes = decompositions + keys read + results written
   mixed_tiles, mixed_graph
                      the benchmark's mixed batch of 1024 negacyclic products (nphi 2048..16384,
-                     k 1..8, seeded draw): one persistent launch, or 3 launches per size group
+                     k 1..8, seeded draw): one persistent launch, or the launches of cp_polymul_list per size group
   bfv_chain, bfv_chain_target, bfv_chain_large
                      the batched BFV multiplication chain (cp_bfv_mul_batch) at nphi 8192 / k 5 /
                      128 pairs, nphi 16384 / k 10 / 32 pairs and nphi 32768 / k 16 / t 65537 / 64
@@ -111,7 +111,7 @@ def workloads():
         e.sample(b, QBase, UNIFORM, 3, P, npolys=P, to_dgt=False)
         ws = e.polymul_workspace(QBase, P)
         return (lambda: e.polymul(c, a, b, QBase, ws, P), 3 * P * 2 * e.N * 16,
-                "fused polymul (3 launches), nphi 4096, k 2, %d polys; bytes = a, b read + c written" % P, e)
+                "fused polymul, nphi 4096, k 2, %d polys; bytes = a, b read + c written" % P, e)
 
     W["polymul"] = polymul
 
@@ -217,7 +217,7 @@ def workloads():
             return (mp.run, mp.algorithmic_bytes(),
                     "mixed batch of 1024 polymuls (nphi 2048..16384, k 1..8), %s" %
                     ("one persistent launch (cp_polymul_tiles)" if mode == "tiles"
-                     else "3 launches per size group (cp_polymul_list)"), e)
+                     else "%d launches (cp_polymul_list per size group)" % mp.launches_per_run()), e)
         return build
 
     W["mixed_tiles"] = mixed("tiles")
