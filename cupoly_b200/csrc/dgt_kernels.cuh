@@ -702,7 +702,7 @@ __global__ void __launch_bounds__(256)
   const ulonglong2* xs = (src_base ? src_base : data) + poly * poly_stride + ((size_t)r << (logNc + S));
   if constexpr (SPREAD) {
     x = fwd_dst(A, data, poly, poly_stride) + ((size_t)r << (logNc + S));
-    xs = src_base ? xs + src_shift(A, poly) : x;
+    xs = src_base ? src_base + poly * poly_stride + src_shift(A, poly) + ((size_t)r << (logNc + S)) : x;
   }
   constexpr int K = 1 << S;
   uint64_t xr[K], xi[K];
